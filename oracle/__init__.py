@@ -62,7 +62,7 @@ def build(ref: bool | None = None) -> None:
     reference tree is present).  Uses oracle/Makefile."""
     subprocess.check_call(["make", "-s", "-C", HERE, "liboracle", "refinputs"])
     if ref is None:
-        ref = os.path.isdir(REFERENCE_TREE)
+        ref = os.path.isfile(os.path.join(REFERENCE_TREE, "src", "kernels.cu"))
     if ref:
         subprocess.check_call(["make", "-s", "-C", HERE, "ref", f"REF={REFERENCE_TREE}"])
 
