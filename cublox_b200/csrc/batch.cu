@@ -7,6 +7,9 @@
 //        ray, the exact walk of ray_walk.cuh), and flushes the cube into the
 //        map's counters.  Points are read in place from one concatenated
 //        x0 y0 z0 x1 ... buffer.
+//        The default shapes order an item's rays by direction instead and
+//        walk 32 neighbouring rays per warp in step, without a cube
+//        (cone_walk.cuh).
 //  fold  persistent CTAs take (map, line range) items; their warps fold the
 //        32-voxel lines the walk flagged, a whole 128-byte line per access
 //        (fold.cuh, fold_lines).
@@ -27,6 +30,7 @@
 #include <vector>
 
 #include "../../include/cublox_b200.h"
+#include "cone_walk.cuh"
 #include "exact_fp.cuh"
 #include "fold.cuh"
 #include "grid_internal.hpp"
@@ -374,78 +378,52 @@ __global__ void __launch_bounds__(512, 2) batch_walk_flat_kernel(const MapDesc *
   }
 }
 
-// Persistent walk without per-item barriers.  A CTA adopts one map at a
-// time (starting at blockIdx % maps, then the next map with rays left): it
-// zeroes its cube around that map's sensor, and its warps take 32-ray items
-// of the map from the map's own counter until none is left; only then does
-// the CTA synchronise, flush the cube and move on.  A warp waits only for
-// its own longest ray, never for the rest of the CTA.  counters[1] holds the
-// number of maps; next[m] is map m's item counter (zero at launch).
-template <int S>
-__global__ void __launch_bounds__(1024) batch_walk_wq_kernel(const MapDesc *maps,
-                                                             const WalkItem * /*items*/,
-                                                             int *counters, int *next) {
-  extern __shared__ uint32_t cube[];
-  constexpr int kCube = S * S * S;
-  __shared__ int s_map;
-  const int n_maps = counters[1];
-  const unsigned lane = threadIdx.x & 31u;
-  int m = n_maps > 0 ? static_cast<int>(blockIdx.x) % n_maps : 0;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      int found = -1;
-      for (int k = 0; k < n_maps; ++k) {
-        const int mm = (m + k) % n_maps;
-        if (*reinterpret_cast<volatile int *>(next + mm) * 32 < maps[mm].ray.n) {
-          found = mm;
-          break;
-        }
-      }
-      s_map = found;
-    }
-    __syncthreads();
-    m = s_map;
-    if (m < 0) break;
-    const MapDesc &md = maps[m];
-    const RayParams p = md.ray;
-    const int clo[3] = {md.clo[0], md.clo[1], md.clo[2]};
-    for (int q = threadIdx.x; q < kCube / 4; q += blockDim.x)
-      reinterpret_cast<uint4 *>(cube)[q] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    uint32_t rays = 0, incs = 0, hits = 0;
-    for (;;) {
-      int it = 0;
-      if (lane == 0) it = atomicAdd(next + m, 1);
-      it = __shfl_sync(0xffffffffu, it, 0);
-      if (it * 32 >= p.n) break;
-      const int i = it * 32 + static_cast<int>(lane);
-      if (i >= p.n) continue;
-      const size_t k = static_cast<size_t>(i) * p.stride;
-      RayWalk w;
-      if (!ray_begin(p, p.x[k], p.y[k], p.z[k], w)) continue;
-      ++rays;
-      const RayEnd re = ray_end_of<S>(p, w, clo);
-      FarWalk f;
-      if (!walk_near<S>(p, cube, clo, w, f, incs)) walk_far(p, f, f.left, incs);
-      apply_end<S>(p, cube, re, incs, hits);
-    }
-    __syncthreads();
-    flush_cube<S>(p, cube, clo);
-    if (p.stats) {
+// One cone walk item (cone_walk.cuh): at most kRays = blockDim.x rays, one a
+// thread, ordered by direction.  `map` is the map whose table is in `table`
+// (-1: none).  Ends with a CTA barrier.
+template <int kRays>
+__device__ __forceinline__ void walk_item_cone(const MapDesc *maps, const WalkItem &item, int *table,
+                                               int &map, ConeItem<kRays> &ci) {
+  const RayParams &p = maps[item.map].ray;
+  if (item.map != map) cone_table(p, table);  // cone_order's barriers follow
+  map = item.map;
+  const int r = cone_order<kRays>(p, item.start, item.count, ci);
+  uint32_t rays = 0, incs = 0, hits = 0;
+  cone_walk(p, table, r >= 0, r >= 0 ? ci.x[r] : 0.0f, r >= 0 ? ci.y[r] : 0.0f,
+            r >= 0 ? ci.z[r] : 0.0f, rays, incs, hits);
+  if (p.stats) {
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        rays += __shfl_down_sync(0xffffffffu, rays, off);
-        incs += __shfl_down_sync(0xffffffffu, incs, off);
-        hits += __shfl_down_sync(0xffffffffu, hits, off);
-      }
-      if (lane == 0) {
-        atomicAdd(p.stats + 0, static_cast<unsigned long long>(rays));
-        atomicAdd(p.stats + 1, static_cast<unsigned long long>(incs));
-        atomicAdd(p.stats + 2, static_cast<unsigned long long>(hits));
-      }
+    for (int off = 16; off > 0; off >>= 1) {
+      rays += __shfl_down_sync(0xffffffffu, rays, off);
+      incs += __shfl_down_sync(0xffffffffu, incs, off);
+      hits += __shfl_down_sync(0xffffffffu, hits, off);
     }
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(p.stats + 0, static_cast<unsigned long long>(rays));
+      atomicAdd(p.stats + 1, static_cast<unsigned long long>(incs));
+      atomicAdd(p.stats + 2, static_cast<unsigned long long>(hits));
+    }
+  }
+  __syncthreads();
+}
+
+// Persistent cone walk: CTAs take items of kRays rays from counters[0].
+template <int kRays>
+__global__ void __launch_bounds__(kRays, 1024 / kRays) batch_walk_cone_kernel(const MapDesc *maps,
+                                                                            const WalkItem *items,
+                                                                            int *counters) {
+  extern __shared__ uint32_t smem[];
+  __shared__ ConeItem<kRays> ci;
+  __shared__ int s_item;
+  int *table = reinterpret_cast<int *>(smem);
+  const int n_items = counters[1];
+  int map = -1;
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(&counters[0], 1);
     __syncthreads();
-    m = (m + 1) % n_maps;
+    const int it = s_item;
+    if (it >= n_items) break;
+    walk_item_cone<kRays>(maps, items[it], table, map, ci);
   }
 }
 
@@ -622,37 +600,38 @@ __global__ void __launch_bounds__(512, 2) batch_fused_flat_kernel(const MapDesc 
 
 struct Shape {
   int cube;      // 0, 16, 32
-  int rays;      // rays per walk item; 0: about two items per resident CTA
+  int rays;      // rays per walk item
   int block;     // walk (or fused) CTA size
   int fused;     // >= 1: one launch, a map's folds queued `fused` maps after its walks
   int min_ctas;  // 2: registers capped for two CTAs per SM (cube <= 16)
-  int wq;        // 1: warps take 32-ray items of a CTA's current map (no item barriers)
   int refill;    // 1: two-phase items, lanes refilled from a far-state queue
   int flat;      // 1: S x S x S/2 cube, two 512-thread CTAs per SM
+  int cone;      // 1: cone walk, one ray a thread in direction order (cone_walk.cuh)
 };
 
-const Shape kShapes[] = {{32, 512, 512, 0, 1, 0, 0},  {32, 1024, 1024, 0, 1, 0, 0},
-                         {32, 0, 512, 0, 1, 1, 0},    {32, 0, 1024, 0, 1, 1, 0},
-                         {16, 0, 512, 0, 1, 1, 0},    {16, 1024, 1024, 0, 2, 0, 0},
-                         {32, 1024, 1024, 1, 1, 0, 0}, {16, 512, 512, 1, 1, 0, 0},
-                         {32, kRefillRays, 512, 0, 1, 0, 1}, {16, kRefillRays, 512, 0, 1, 0, 1},
-                         {32, 512, 512, 0, 2, 0, 0, 1},     {32, 256, 512, 0, 2, 0, 0, 1},
-                         {32, 512, 512, 2, 2, 0, 0, 1},     {32, 512, 512, 1, 2, 0, 0, 1},
-                         {32, 1024, 512, 0, 2, 0, 0, 1},    {32, 768, 512, 0, 2, 0, 0, 1}};
+const Shape kShapes[] = {{0, 512, 512, 0, 1, 0, 0, 1},          {32, 1024, 1024, 0, 1, 0, 0, 0},
+                         {0, 256, 256, 0, 1, 0, 0, 1},          {0, 1024, 1024, 0, 1, 0, 0, 1},
+                         {32, 512, 512, 0, 1, 0, 0, 0},         {16, 1024, 1024, 0, 2, 0, 0, 0},
+                         {32, 1024, 1024, 1, 1, 0, 0, 0},       {16, 512, 512, 1, 1, 0, 0, 0},
+                         {32, kRefillRays, 512, 0, 1, 1, 0, 0}, {16, kRefillRays, 512, 0, 1, 1, 0, 0},
+                         {32, 512, 512, 0, 2, 0, 1, 0},         {32, 256, 512, 0, 2, 0, 1, 0},
+                         {32, 512, 512, 2, 2, 0, 1, 0},         {32, 512, 512, 1, 2, 0, 1, 0},
+                         {32, 1024, 512, 0, 2, 0, 1, 0},        {32, 768, 512, 0, 2, 0, 1, 0}};
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
+constexpr int kWideShape = 10;  // walks the maps that the cone walk does not take (cone_takes)
 
-// The tuner's candidates: the launch shapes that have been fastest on some
-// workload, with the default voxel layout (8 x 4 x 1 bricks), then the two
-// fastest walk shapes with the other layouts (4 x 8 x 1 and 4 x 4 x 2
-// bricks, the reference's hash order).  Shapes 3, 4, 5, 8, 9 and 13 stay
-// selectable.  A candidate with another layout moves every grid of the
-// update to it first.
+// The tuner's candidates: the cone walk's item sizes with the default voxel
+// layout (8 x 4 x 1 bricks), its usual size with 4 x 8 x 1 and 4 x 4 x 2
+// bricks, and the fastest of the shapes with a counter cube.  The cone walk
+// has been the fastest on every workload measured (8 README-scale maps: 0.64
+// ms against 1.16 ms for shape 10; 32 maps of three sizes: 1.16 against 3.19),
+// so the other shapes and the reference's hash order are no longer timed;
+// all stay selectable.  A candidate with another layout moves every grid of
+// the update to it first.
 struct Candidate {
   int shape, layout;
 };
-const Candidate kCandidates[] = {{0, 320},  {1, 320},  {2, 320},  {6, 320},  {7, 320},
-                                 {10, 320}, {11, 320}, {12, 320}, {14, 320}, {15, 320},
-                                 {1, 230},  {10, 230}, {1, 221},  {10, 221}, {1, 0}};
+const Candidate kCandidates[] = {{0, 320}, {2, 320}, {3, 320}, {0, 230}, {0, 221}, {10, 320}};
 constexpr int kNumCandidates = sizeof(kCandidates) / sizeof(kCandidates[0]);
 
 int sm_count_batch() {
@@ -672,7 +651,6 @@ const void *shape_kernel_s(const Shape &sh) {
   if (sh.flat) return reinterpret_cast<const void *>(batch_walk_flat_kernel<S>);
   if (sh.refill) return reinterpret_cast<const void *>(batch_walk_refill_kernel<S>);
   if (sh.fused) return reinterpret_cast<const void *>(batch_fused_kernel<S>);
-  if (sh.wq) return reinterpret_cast<const void *>(batch_walk_wq_kernel<S>);
   if constexpr (S < 32) {
     if (sh.min_ctas >= 2) return reinterpret_cast<const void *>(batch_walk_kernel<S, 2>);
   }
@@ -681,11 +659,16 @@ const void *shape_kernel_s(const Shape &sh) {
 
 // The walk (or fused) kernel of a shape.
 const void *shape_kernel(const Shape &sh) {
+  if (sh.cone)
+    return sh.block == 1024  ? reinterpret_cast<const void *>(batch_walk_cone_kernel<1024>)
+           : sh.block == 512 ? reinterpret_cast<const void *>(batch_walk_cone_kernel<512>)
+                             : reinterpret_cast<const void *>(batch_walk_cone_kernel<256>);
   return sh.cube >= 32 ? shape_kernel_s<32>(sh)
                        : (sh.cube >= 16 ? shape_kernel_s<16>(sh) : shape_kernel_s<0>(sh));
 }
 
 size_t shape_smem(const Shape &sh) {
+  if (sh.cone) return sizeof(int) * kConeTableMax;
   return sizeof(uint32_t) * (sh.cube * sh.cube * (sh.flat ? sh.cube / 2 : sh.cube) +
                              (sh.refill ? kRefillRays * kFarWords : 0));
 }
@@ -699,7 +682,7 @@ int shape_grid(int shape) {
     const Shape &sh = kShapes[shape];
     const void *fn = shape_kernel(sh);
     const size_t smem = shape_smem(sh);
-    if (smem > 48 * 1024 &&
+    if (smem > 16 * 1024 &&  // the cone walk's static shared memory comes on top
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(smem)) != cudaSuccess)
       cudaGetLastError();
@@ -714,23 +697,13 @@ int shape_grid(int shape) {
   return cached[shape];
 }
 
-// Rays per walk item of a shape for a step of `total` rays.
-int shape_rays(int shape, int64_t total) {
-  const Shape &sh = kShapes[shape];
-  if (sh.rays > 0) return sh.rays;
-  const int64_t items = 2 * static_cast<int64_t>(shape_grid(shape));
-  const int64_t per = (total + items - 1) / items;
-  return static_cast<int>(std::min<int64_t>(1 << 20, std::max<int64_t>(256, (per + 31) & ~31)));
-}
-
 cudaError_t launch_walk(const MapDesc *maps, const WalkItem *witems, const FoldItem *fitems,
                         int *counters, int *done, int shape, cudaStream_t s) {
   const Shape &sh = kShapes[shape];
   void *walk_args[] = {&maps, &witems, &counters};
   void *fused_args[] = {&maps, &witems, &fitems, &counters, &done};
-  void *wq_args[] = {&maps, &witems, &counters, &done};
   return cudaLaunchKernel(shape_kernel(sh), dim3(shape_grid(shape)), dim3(sh.block),
-                          sh.fused ? fused_args : (sh.wq ? wq_args : walk_args), shape_smem(sh),
+                          sh.fused ? fused_args : walk_args, shape_smem(sh),
                           s);
 }
 
@@ -886,7 +859,7 @@ cudaError_t enqueue_step(cublox_batch *b, int shape, const char **what) {
       (e = cudaMemsetAsync(b->d_counters + 2, 0, sizeof(int), b->stream)) != cudaSuccess ||
       (e = cudaMemsetAsync(b->d_counters + 4, 0, sizeof(int), b->stream)) != cudaSuccess)
     return e;
-  if ((sh.fused || sh.wq) &&
+  if (sh.fused &&
       (e = cudaMemsetAsync(b->d_done, 0, sizeof(int) * b->maps_cap, b->stream)) != cudaSuccess)
     return e;
   *what = "timing event";
@@ -1066,7 +1039,10 @@ int cublox_batch_update(cublox_batch *b, int n, cublox_grid *const *grids, const
   if (total <= 0) return CUBLOX_OK;  // every scan empty: nothing changes
   const bool tuning = b->autotune && b->tune_step < kNumCandidates * b->tune_rounds;
   const int cand = tuning ? (b->tune_step / b->tune_rounds) % kNumCandidates : -1;
-  const int active_shape = tuning ? kCandidates[cand].shape : b->shape;
+  int active_shape = tuning ? kCandidates[cand].shape : b->shape;
+  if (kShapes[active_shape].cone)
+    for (int i = 0; i < n; ++i)
+      if (!cone_takes(grids[i]->map, grids[i]->nalloc)) active_shape = kWideShape;
   const int active_layout = tuning ? kCandidates[cand].layout : b->layout;
   // the grids' voxel layout (moved between scans, on the batch's stream)
   for (int i = 0; i < n; ++i) {
@@ -1075,7 +1051,7 @@ int cublox_batch_update(cublox_batch *b, int n, cublox_grid *const *grids, const
     if (rc) return rc;
   }
   const Shape &sh = kShapes[active_shape];
-  const int rays_per_item = shape_rays(active_shape, total);
+  const int rays_per_item = sh.rays;
   // work items
   int n_w = 0, n_f = 0;
   for (int i = 0; i < n; ++i) {
@@ -1188,7 +1164,7 @@ int cublox_batch_update(cublox_batch *b, int n, cublox_grid *const *grids, const
   }
   b->h_counters[0] = b->h_counters[2] = b->h_counters[4] = 0;
   b->h_counters[5] = b->wait_limit;
-  b->h_counters[1] = sh.wq ? d : w;  // the warp-queue walk reads maps, not items
+  b->h_counters[1] = w;
   b->h_counters[3] = f;
   cudaError_t e;
   if ((e = cudaMemcpyAsync(b->d_maps, b->h_maps, sizeof(MapDesc) * d, cudaMemcpyHostToDevice,

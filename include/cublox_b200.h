@@ -299,9 +299,10 @@ typedef struct cublox_batch cublox_batch;
 #define CUBLOX_BATCH_OPT_AUTOTUNE 2   /* choose the launch shape and the
                                          voxel layout over the first
                                          updates (default 1): each candidate
-                                         (every shape with 8 x 4 x 1
-                                         bricks, the flat-cube shape with
-                                         the other layouts) is timed twice  */
+                                         (the walk in direction order with
+                                         each item size and brick layout,
+                                         the flat-cube shape) is timed
+                                         twice                              */
 #define CUBLOX_BATCH_OPT_SHAPE 3      /* fix the launch shape (0 .. n-1)    */
 #define CUBLOX_BATCH_OPT_TIMING 4     /* record walk/fold device times      */
 #define CUBLOX_BATCH_OPT_NUM_SHAPES 5 /* read only: number of shapes        */
