@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "../../include/cublox_b200.h"
+#include "cone_walk.cuh"
 #include "exact_fp.cuh"
 #include "grid_internal.hpp"
 #include "kernels.cuh"
@@ -594,7 +595,16 @@ static int ensure_stage(cublox_grid *g, int n) {
   return CUBLOX_OK;
 }
 
-// Launch raycast (+ fold unless count_only) on a device SoA cloud.
+// The default walk goes in direction order (cone_walk.cuh), about twice as
+// fast as the split walk at every size measured (raycast_cone.cu), unless the
+// map is too wide for it or an option of the split walk was set.
+static bool walks_cones(const cublox_grid *g) {
+  return g->opt_raycast == 2 && g->opt_cube == 32 && !g->opt_flat && !g->opt_sort &&
+         g->opt_seg == 64 && g->opt_block == 512 && !g->opt_contig &&
+         cone_takes(g->map, g->nalloc);
+}
+
+// Launch raycast (+ fold unless count_only) on a device cloud.
 static int integrate(cublox_grid *g, const float *dx, const float *dy,
                      const float *dz, int n, int stride,
                      const float sensor[3], bool count_only = false) {
@@ -643,7 +653,9 @@ static int integrate(cublox_grid *g, const float *dx, const float *dy,
     g->bin_cap = n;
   }
   tmark(g, 0, 0);
-  if (g->opt_raycast == 2 && p.stride != 1) {
+  const bool cone = walks_cones(g);
+  const bool split = g->opt_raycast == 2 && !cone;
+  if (split && p.stride != 1) {
     // the split walk reads SoA: gather an AoS cloud first
     int rc = ensure_cloud(g, n);
     if (rc) return rc;
@@ -657,7 +669,7 @@ static int integrate(cublox_grid *g, const float *dx, const float *dy,
     }
   }
   constexpr int kMaxSegsPerRay = 16;
-  if (g->opt_raycast == 2 && (n > g->split_cap || !g->d_work)) {
+  if (split && (n > g->split_cap || !g->d_work)) {
     CK(cudaStreamSynchronize(g->stream));
     cublox_b200::detail::dfree(g->d_segs);
     cublox_b200::detail::dfree(g->d_rays);
@@ -673,7 +685,9 @@ static int integrate(cublox_grid *g, const float *dx, const float *dy,
     }
     g->split_cap = n;
   }
-  if (g->opt_raycast == 2) {
+  if (cone) {
+    launch_raycast_cone(p, g->stream);
+  } else if (split) {
     SplitScratch sc{g->d_segs, g->d_rays, g->d_work, kMaxSegsPerRay * n, kMaxSegsPerRay,
                     g->opt_block, g->opt_contig};
     RayParams ps = p;
@@ -901,7 +915,10 @@ static int update_impl(cublox_grid *g, const float *x, const float *y,
   CK(cudaEventSynchronize(g->stage_ev[s]));
   float *h = g->h_stage[s];
   const size_t nb = sizeof(float) * static_cast<size_t>(n);
-  if (xyz && layout == CUBLOX_LAYOUT_AOS) {
+  const bool as_is = xyz && layout == CUBLOX_LAYOUT_AOS && walks_cones(g);  // reads any stride
+  if (as_is) {
+    std::memcpy(h, xyz, 3 * nb);
+  } else if (xyz && layout == CUBLOX_LAYOUT_AOS) {
     for (int i = 0; i < n; ++i) {
       h[i] = xyz[3 * static_cast<size_t>(i)];
       h[n + i] = xyz[3 * static_cast<size_t>(i) + 1];
@@ -916,6 +933,7 @@ static int update_impl(cublox_grid *g, const float *x, const float *y,
   }
   CK(cudaMemcpyAsync(g->d_cloud, h, 3 * nb, cudaMemcpyHostToDevice, g->stream));
   CK(cudaEventRecord(g->stage_ev[s], g->stream));
+  if (as_is) return integrate(g, g->d_cloud, g->d_cloud + 1, g->d_cloud + 2, n, 3, sensor);
   return integrate(g, g->d_cloud, g->d_cloud + n, g->d_cloud + 2 * static_cast<size_t>(n), n,
                    1, sensor);
 }

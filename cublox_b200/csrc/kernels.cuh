@@ -177,6 +177,9 @@ size_t split_ray_bytes();
 // 32 only): a 32 x 32 x 16 cube, two CTAs per SM.
 void launch_raycast_split(const RayParams &p, int cube, bool flat, int seg_len,
                           const SplitScratch &sc, cudaStream_t s);
+// Walk in direction order (raycast_cone.cu), for maps that cone_takes
+// (cone_walk.cuh) and points of any stride.
+void launch_raycast_cone(const RayParams &p, cudaStream_t s);
 // cube: side of the shared-memory counter cube (16 or 32); match: merge
 // duplicate voxel keys within a warp; sort: walk rays in direction order.
 void launch_raycast_binned(const RayParams &p, const BinnedScratch &b, int cube,

@@ -92,3 +92,32 @@ def test_map_too_wide_for_the_step_table():
     s = np.float32([[0.0, 0.0, 0.0]])
     _check(g, half, False, s, [_clouds(rng, 2000, s[0])], lambda p, x: b.update([g], [p], [x]))
     b.close()
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 4096, 32767, 32769, 65537, 131073])
+@pytest.mark.parametrize("source", ["host", "device", "device_soa"])
+def test_single_grid_items(n, source):
+    """One grid's update at the sizes where its items get wider."""
+    import torch
+
+    half, rng = (40, 33, 14), np.random.default_rng(n)
+    g = C.OccupancyGrid(half, 0.1, False, 1.0)
+    g.setLogOddsParams(*LO)
+    g.setMaxRaycastRange(6.0)
+    sensors = np.float32([[0.03, -0.02, 0.41], [1.9, -1.4, 0.6]])
+    keep = []
+
+    def update(p, s):
+        if source != "host":
+            t = torch.from_numpy(p).cuda()
+            keep.append(t if source == "device" else t.T.contiguous())
+            torch.cuda.synchronize()
+            if source == "device":
+                g.update_ptr(keep[-1].data_ptr(), n, s, C.LAYOUT_AOS)
+            else:
+                g.update_ptr(keep[-1].data_ptr(), n, s, C.LAYOUT_SOA)
+        else:
+            g.update(p, s)
+
+    _check(g, half, False, sensors, [_clouds(rng, n, s) for s in sensors], update)
+    g.close()
