@@ -326,7 +326,7 @@ template <bool kL2, bool kAll = false>
 __device__ __forceinline__ uint32_t fold_item(const MapDesc &m, const FoldItem &item) {
   const FoldView v = fold_view(m);
   const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  return fold_lines<8, kL2, kAll>(v, m.ray.dirty, item.start + 32 * warp, item.start + item.count,
+  return fold_lines<8, kL2, kAll>(v, m.ray.dirty, m.ray.hot, item.start + 32 * warp, item.start + item.count,
                                   32 * warps);
 }
 
@@ -448,42 +448,27 @@ __global__ void __launch_bounds__(256) batch_fold_kernel(const MapDesc *maps,
 }
 
 // Persistent fold over per-item lists of the flagged lines (fold.cuh,
-// build_line_list / fold_line_list): CTAs take fold items from counters[2]
-// and load the next item's flags before folding the current list.
+// build_line_list / fold_line_list): CTAs take fold items from counters[2].
+// An item's flags are not loaded ahead of the fold before it: the registers
+// they would hold spill (8 maps 0.457 ms, against 0.452).
 template <int kQuads, int kMinCtas>
 __global__ void __launch_bounds__(kListThreads, kMinCtas) batch_fold_list_kernel(
     const MapDesc *maps, const FoldItem *items, int *counters) {
   __shared__ LineList L;
-  __shared__ HitQueue hq;
   __shared__ int s_item;
   const int n_items = counters[3];
-  if (threadIdx.x == 0) {
-    s_item = atomicAdd(&counters[2], 1);
-    hq.n = 0;
-  }
-  __syncthreads();
-  int it = s_item;
-  uint4 f = make_uint4(0u, 0u, 0u, 0u);
-  if (it < n_items) {
-    const FoldItem fi = items[it];
-    f = load_line_flags(maps[fi.map].ray.dirty, fi.start, fi.count);
-  }
-  while (it < n_items) {
-    const FoldItem item = items[it];
-    const MapDesc &m = maps[item.map];
-    const int n = build_line_list(line_flag_bits(f), L, m.ray.dirty, item.start, item.count);
+  for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(&counters[2], 1);
     __syncthreads();
-    const int next = s_item;
-    if (next < n_items) {
-      const FoldItem fi = items[next];
-      f = load_line_flags(maps[fi.map].ray.dirty, fi.start, fi.count);
-    }
-    const FoldView v = fold_view(m);
-    add_touched(m, fold_line_list<kQuads, false>(v, L.line, n, item.start, &hq));
-    __syncthreads();
-    fold_hit_queue(v, hq);  // ends with a barrier: the list and s_item are rewritten next
-    it = next;
+    if (s_item >= n_items) break;
+    const FoldItem item = items[s_item];
+    const MapDesc &m = maps[item.map];
+    const uint4 f = load_line_flags(m.ray.dirty, item.start, item.count);
+    const uint4 fh = load_line_flags(m.ray.hot, item.start, item.count);
+    const int2 n = build_line_list(line_flag_bits(f), line_flag_bits(fh), L, m.ray.dirty, m.ray.hot,
+                                   item.start, item.count);
+    add_touched(m, fold_line_list<kQuads, false>(fold_view(m), L, n, item.start));
+    __syncthreads();  // the list and s_item are rewritten next
   }
 }
 
@@ -564,9 +549,7 @@ __global__ void __launch_bounds__(512, 2) batch_fused_flat_kernel(const MapDesc 
                                                                   int *counters, int *done) {
   extern __shared__ uint32_t cube[];
   __shared__ LineList L;
-  __shared__ HitQueue hq;
   __shared__ int s_item, s_ok;
-  if (threadIdx.x == 0) hq.n = 0;
   const int n_all = counters[1];
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(&counters[0], 1);
@@ -587,11 +570,10 @@ __global__ void __launch_bounds__(512, 2) batch_fused_flat_kernel(const MapDesc 
       __syncthreads();
       if (s_ok) {
         const uint4 f = load_line_flags<true>(m.ray.dirty, item.start, item.count);
-        const int n = build_line_list(line_flag_bits(f), L, m.ray.dirty, item.start, item.count);
-        const FoldView v = fold_view(m);
-        add_touched(m, fold_line_list<2, true>(v, L.line, n, item.start, &hq));
-        __syncthreads();
-        fold_hit_queue(v, hq);
+        const uint4 fh = load_line_flags<true>(m.ray.hot, item.start, item.count);
+        const int2 n = build_line_list(line_flag_bits(f), line_flag_bits(fh), L, m.ray.dirty, m.ray.hot,
+                                      item.start, item.count);
+        add_touched(m, fold_line_list<2, true>(fold_view(m), L, n, item.start));
       }
       __syncthreads();
     }
@@ -711,7 +693,9 @@ cudaError_t launch_fold(const MapDesc *maps, const FoldItem *fitems, int *counte
                         int variant, cudaStream_t s) {
   const dim3 grid(sm_count_batch() * 8), block(256);
   if (variant == 0) {
-    batch_fold_list_kernel<4, 4><<<sm_count_batch() * 4, kListThreads, 0, s>>>(maps, fitems, counters);
+    // three accesses in flight a warp: a fourth spills at four CTAs per SM
+    // (8 maps 0.64 ms, against 0.45), and two, at five or six, spill too
+    batch_fold_list_kernel<3, 4><<<sm_count_batch() * 4, kListThreads, 0, s>>>(maps, fitems, counters);
   } else if (variant == 1) {
     batch_fold_kernel<true><<<grid, block, 0, s>>>(maps, fitems, counters);
   } else {

@@ -264,7 +264,7 @@ int64_t cublox_b200::detail::nalloc_for(const int half[3]) {
 
 size_t cublox_b200::detail::voxel_bytes_for(const int half[3]) {
   const int64_t nalloc = nalloc_for(half);
-  return 12 * static_cast<size_t>(nalloc) + static_cast<size_t>(nalloc >> kLineShift);
+  return 12 * static_cast<size_t>(nalloc) + 2 * flag_bytes(static_cast<int>(nalloc >> kLineShift));
 }
 
 bool cublox_b200::detail::layout_valid(int code) {
@@ -398,8 +398,8 @@ int cublox_grid_create(const int half_map_size[3], float resolution,
     g->own_stream = true;
   }
   const size_t n = static_cast<size_t>(g->nalloc);
-  if ((e = cublox_b200::detail::dmalloc(&g->d_dirty, static_cast<size_t>(g->nlines))) != cudaSuccess) return bail(e, "cudaMalloc line flags");
-  if ((e = cudaMemsetAsync(g->d_dirty, 0, static_cast<size_t>(g->nlines), g->stream)) != cudaSuccess) return bail(e, "memset line flags");
+  if ((e = cublox_b200::detail::dmalloc(&g->d_dirty, 2 * flag_bytes(g->nlines))) != cudaSuccess) return bail(e, "cudaMalloc line flags");
+  if ((e = cudaMemsetAsync(g->d_dirty, 0, 2 * flag_bytes(g->nlines), g->stream)) != cudaSuccess) return bail(e, "memset line flags");
   if ((e = cublox_b200::detail::dmalloc(&g->d_occ, n * sizeof(float))) != cudaSuccess) return bail(e, "cudaMalloc occ");
   if ((e = cublox_b200::detail::dmalloc(&g->d_cnt, n * sizeof(uint32_t))) != cudaSuccess) return bail(e, "cudaMalloc cnt");
   if ((e = cublox_b200::detail::dmalloc(&g->d_hit, n * sizeof(uint32_t))) != cudaSuccess) return bail(e, "cudaMalloc hit");
@@ -443,7 +443,7 @@ int cublox_grid_reset(cublox_grid *g) {
   CK(cudaMemsetAsync(g->d_occ, 0, n * sizeof(float), g->stream));
   CK(cudaMemsetAsync(g->d_cnt, 0, n * sizeof(uint32_t), g->stream));
   CK(cudaMemsetAsync(g->d_hit, 0, n * sizeof(uint32_t), g->stream));
-  CK(cudaMemsetAsync(g->d_dirty, 0, static_cast<size_t>(g->nlines), g->stream));
+  CK(cudaMemsetAsync(g->d_dirty, 0, 2 * flag_bytes(g->nlines), g->stream));
   CK(cudaStreamSynchronize(g->stream));
   g->first_run = true;
   return CUBLOX_OK;
@@ -634,6 +634,7 @@ static int integrate(cublox_grid *g, const float *dx, const float *dy,
   p.err = g->d_err;
   p.lay = g->lay;
   p.dirty = g->d_dirty;
+  p.hot = g->d_dirty + flag_bytes(g->nlines);
   if ((g->opt_raycast == 1 || (g->opt_raycast == 2 && g->opt_sort)) && n > g->bin_cap) {
     CK(cudaStreamSynchronize(g->stream));
     cublox_b200::detail::dfree(g->d_bins);
@@ -723,6 +724,7 @@ static int integrate(cublox_grid *g, const float *dx, const float *dy,
   a.stats = g->stats_on ? g->d_stats : nullptr;
   a.variant = g->opt_fold;
   a.dirty = g->d_dirty;
+  a.hot = g->d_dirty + flag_bytes(g->nlines);
   a.nlines = g->nlines;
   a.err = g->d_err;
   a.vnum = static_cast<int>(std::min<int64_t>(g->nalloc, std::numeric_limits<int>::max()));
@@ -731,7 +733,7 @@ static int integrate(cublox_grid *g, const float *dx, const float *dy,
   CK_LAUNCH();
   // the full sweeps leave the line flags set: clear them
   if (a.variant < 2)
-    CK(cudaMemsetAsync(g->d_dirty, 0, static_cast<size_t>(g->nlines), g->stream));
+    CK(cudaMemsetAsync(g->d_dirty, 0, 2 * flag_bytes(g->nlines), g->stream));
   tmark(g, 1, 1);
   return CUBLOX_OK;
 }
@@ -773,11 +775,12 @@ RayParams cublox_b200::detail::ray_params(const cublox_grid *g, const float *x,
   p.err = g->d_err;
   p.lay = g->lay;
   p.dirty = g->d_dirty;
+  p.hot = g->d_dirty + flag_bytes(g->nlines);
   return p;
 }
 
 size_t cublox_b200::detail::device_bytes(const cublox_grid *g) {
-  size_t b = 12 * static_cast<size_t>(g->d_occ ? g->nalloc : 0) + static_cast<size_t>(g->nlines);
+  size_t b = 12 * static_cast<size_t>(g->d_occ ? g->nalloc : 0) + 2 * flag_bytes(g->nlines);
   b += sizeof(float) * 3 * (static_cast<size_t>(g->cloud_cap) + static_cast<size_t>(g->world_cap));
   b += g->image_cap;
   b += g->fs.fq_bytes + 13 * static_cast<size_t>(g->fs.fcap) + 13 * static_cast<size_t>(g->qcap);
@@ -1824,7 +1827,7 @@ int cublox_grid_count_scan(cublox_grid *g, const float *xyz, int n,
   CK(cudaMemcpyAsync(hh.data(), g->d_hit, ab, cudaMemcpyDeviceToHost, g->stream));
   CK(cudaMemsetAsync(g->d_cnt, 0, ab, g->stream));
   CK(cudaMemsetAsync(g->d_hit, 0, ab, g->stream));
-  CK(cudaMemsetAsync(g->d_dirty, 0, static_cast<size_t>(g->nlines), g->stream));
+  CK(cudaMemsetAsync(g->d_dirty, 0, 2 * flag_bytes(g->nlines), g->stream));
   CK(cudaStreamSynchronize(g->stream));
   for (int h = 0; h < g->voxel_num; ++h) {
     const int a = hash_addr(g, h);

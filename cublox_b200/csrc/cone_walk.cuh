@@ -313,8 +313,7 @@ __device__ __forceinline__ void cone_walk(const RayParams &p, const int *table, 
     p.dirty[r.he >> kLineShift] = 1;
     ++incs;
     if (hit) {
-      atomicOr(p.cnt + r.he, kHitFlag);
-      red_add(p.hit + r.he, 1u);
+      mark_hit(p, r.he, 1u);
       ++hits;
     }
   }

@@ -79,8 +79,7 @@ __device__ __forceinline__ void apply_end(const RayParams &p, uint32_t *cube, co
   }
   ++incs;
   if (r.hit) {
-    atomicOr(p.cnt + r.h, kHitFlag);
-    atomicAdd(p.hit + r.h, 1u);
+    mark_hit(p, r.h, 1u);
     ++hits;
   }
 }

@@ -97,8 +97,8 @@ __device__ __forceinline__ uint32_t fold_groups(const FoldView &v, int first, in
 // lines.  kL2: flags and counters are read at L2 (ld.global.cg), as a launch
 // that also wrote them from other CTAs needs.  Returns the voxels folded.
 template <int kLines, bool kL2, bool kAll = false>
-__device__ __forceinline__ uint32_t fold_lines(const FoldView &v, uint8_t *dirty, int first,
-                                               int end, int stride) {
+__device__ __forceinline__ uint32_t fold_lines(const FoldView &v, uint8_t *dirty, uint8_t *hot,
+                                               int first, int end, int stride) {
   const int lane = threadIdx.x & 31;
   uint32_t touched = 0;
   auto flag = [&](int l) -> bool {
@@ -109,7 +109,7 @@ __device__ __forceinline__ uint32_t fold_lines(const FoldView &v, uint8_t *dirty
     const int l = base + lane;
     const bool d = next;
     uint32_t mask = __ballot_sync(0xffffffffu, d);
-    if (d) dirty[l] = 0;
+    if (d) dirty[l] = hot[l] = 0;
     next = flag(base + stride + lane);
     while (mask) {
       int at[kLines];
@@ -145,23 +145,30 @@ __device__ __forceinline__ uint32_t fold_lines(const FoldView &v, uint8_t *dirty
 }
 
 // ---- flagged lines compacted into a list per CTA ----
-// The per-warp fold above reads 32 flags, then folds only the flagged ones
-// among them: about 9 of 32 lines at README scale, so a warp rarely has more
-// than one batch of lines in flight and waits a full memory latency on every
-// flag group.  Here a CTA (256 threads or more) takes up to 4096 lines at a
-// time: one 16-byte flag load for each of its first 256 threads, a CTA-wide
-// prefix sum turns the flagged lines into a
-// dense list in shared memory (flags cleared on the way), and the warps then
-// fold the list four lines per warp access (8 lanes x 16 bytes a line) with
-// kQuads accesses in flight per warp, so every warp has 4 kQuads lines in
-// flight until the list runs out.  The next item's flags are loaded before
-// the current list is folded.
+// The fold is bound by HBM: 256 bytes read and up to 256 written per flagged
+// line, at scattered 128-byte lines (5.3 TB/s for the bare access pattern;
+// the fold moves about 278 MB in 58 us for one README-scale scan and in 57 us
+// a map for eight, 4.8 TB/s; 74 and 64 us before lines with a hit had a flag
+// of their own).  The per-warp fold above reads 32 flags, then folds only the
+// flagged ones among them: about 9 of 32 lines at README scale, so a warp
+// rarely has more than one batch of lines in flight and waits a full memory
+// latency on every flag group.  Here a CTA (256 threads or more) takes up to
+// 4096 lines at a time: one 16-byte flag load for each of its first 256
+// threads, a CTA-wide prefix sum turns the flagged lines into a dense list in
+// shared memory (flags cleared on the way), and the warps then fold the list
+// four lines per warp access (8 lanes x 16 bytes a line) with kQuads accesses
+// in flight per warp.  Lines with a hit (3 in 100) make a list of their own,
+// folded with the hit counts loaded beside the counters: queueing their
+// voxels for the end of the item cost two barriers and two more round trips
+// to memory per item.
 
 constexpr int kListThreads = 256;              // CTA size of the fold-only kernels
 constexpr int kListLines = 16 * kListThreads;  // lines per item: 16 flags per thread
 
 struct LineList {
-  uint16_t line[kListLines];  // flagged lines, relative to the item's first line
+  // flagged lines, relative to the item's first line: without a hit from the
+  // front, with one from the back
+  uint16_t line[kListLines];
   int warp_sum[32];
 };
 
@@ -197,13 +204,27 @@ __device__ __forceinline__ uint32_t line_flag_bits(const uint4 &f) {
   return m;
 }
 
-// The CTA's list from every thread's flag bits `m` (item of `count` lines
-// from line `start`); clears the flags it found.  Returns the list's
-// length.  Contains two CTA barriers, the last at the end.
-__device__ __forceinline__ int build_line_list(uint32_t m, LineList &L, uint8_t *dirty, int start,
-                                               int count) {
+// Clears the flags of this thread's lines start + 16 t .. + 15 that are set
+// in `m`.
+__device__ __forceinline__ void clear_line_flags(uint32_t m, uint8_t *flags, int start, int count) {
+  const int i = 16 * static_cast<int>(threadIdx.x);
+  if (!m) return;
+  if (i + 16 <= count)  // the thread's 16 flags are one aligned 16-byte word
+    *reinterpret_cast<uint4 *>(flags + start + i) = make_uint4(0u, 0u, 0u, 0u);
+  else
+    for (uint32_t r = m; r; r &= r - 1) flags[start + i + __ffs(r) - 1] = 0;
+}
+
+// The CTA's list from every thread's flag bits `m`, and `hot` of the lines
+// with a hit (item of `count` lines from line `start`); clears the flags it
+// found.  Returns the lines without a hit (x) and with one (y).  Contains
+// two CTA barriers, the last at the end.
+__device__ __forceinline__ int2 build_line_list(uint32_t m, uint32_t hot, LineList &L,
+                                                uint8_t *dirty, uint8_t *hot_flags, int start,
+                                                int count) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = __popc(m);
+  const uint32_t cold = m & ~hot;
+  const int c = __popc(cold) | __popc(hot) << 16;  // both sums at once
   int incl = c;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -220,61 +241,31 @@ __device__ __forceinline__ int build_line_list(uint32_t m, LineList &L, uint8_t 
     total += s;
   }
   const int i = 16 * static_cast<int>(threadIdx.x);
-  for (uint32_t r = m; r; r &= r - 1) L.line[pos++] = static_cast<uint16_t>(i + __ffs(r) - 1);
-  if (m) {
-    if (i + 16 <= count)  // the thread's 16 flags are one aligned 16-byte word
-      *reinterpret_cast<uint4 *>(dirty + start + i) = make_uint4(0u, 0u, 0u, 0u);
-    else
-      for (uint32_t r = m; r; r &= r - 1) dirty[start + i + __ffs(r) - 1] = 0;
-  }
+  uint16_t *front = L.line + (pos & 0xffff), *back = L.line + kListLines - 1 - (pos >> 16);
+  for (uint32_t r = cold; r; r &= r - 1) *front++ = static_cast<uint16_t>(i + __ffs(r) - 1);
+  for (uint32_t r = hot; r; r &= r - 1) *back-- = static_cast<uint16_t>(i + __ffs(r) - 1);
+  clear_line_flags(m, dirty, start, count);
+  clear_line_flags(hot, hot_flags, start, count);
   __syncthreads();
-  return total;
+  return make_int2(total & 0xffff, total >> 16);
 }
 
-// Voxels with a hit whose fold waits for the end of the item.  Their hit
-// count lives in a second array; loaded where the voxel is met, it would
-// stall the warp's whole batch of lines for one more memory round trip
-// (most batches hold a hit voxel), so they are queued in shared memory
-// and folded together once the list is done, every hit load in flight at
-// once.  A full queue folds further hits where they are met.
-constexpr int kHitCap = 1024;
-
-struct HitQueue {
-  int n;                 // voxels queued (may pass kHitCap: the rest were folded in place)
-  int h[kHitCap];        // address
-  uint32_t c[kHitCap];   // counter word
-};
-
-// Folds voxel h (counter word c, stored value o) now, or queues it if it has
-// a hit and the queue has room (its stored value is then written back
-// unchanged by the caller and replaced by fold_hit_queue).
-__device__ __forceinline__ float fold_or_queue(const FoldView &v, HitQueue *hq, int h, uint32_t c,
-                                               float o) {
-  if (hq && (c & kHitFlag)) {
-    const int slot = atomicAdd(&hq->n, 1);
-    if (slot < kHitCap) {
-      hq->h[slot] = h;
-      hq->c[slot] = c;
-      return o;
-    }
-  }
-  return fold_counter(v, h, c, o);
-}
-
-// Fold of the CTA's list of n lines (relative to line `start`).  Warp w of
-// W takes line quads w, w + W, ...; lane (q, s) = (lane / 8, lane % 8)
-// handles 16-byte piece s of the quad's line q.  A piece whose counters are
-// all zero is left as it is (its values do not change, its counters are
-// zero already).  Hit voxels go to `hq` when it is given (fold_hit_queue
-// folds them after a CTA barrier).  kL2: counters are read at L2.  Returns
-// the voxels folded or queued.
-template <int kQuads, bool kL2>
-__device__ __forceinline__ uint32_t fold_line_list(const FoldView &v, const uint16_t *list, int n,
-                                                   int start, HitQueue *hq = nullptr) {
+// Fold of n lines of the CTA's list (relative to line `start`): kHot, those
+// with a hit, else those without.  Warp w of W takes line quads w, w + W,
+// ...; lane (q, s) = (lane / 8, lane % 8) handles 16-byte piece s of the
+// quad's line q.  A piece whose counters are all zero is left as it is (its
+// values do not change, its counters are zero already).  The hit counts, in
+// an array of their own, are read together with the counters and stored
+// values, and only for lines with a hit.  kL2: counters and hit counts are
+// read at L2.  Returns the voxels folded.
+template <int kQuads, bool kL2, bool kHot>
+__device__ __forceinline__ uint32_t fold_lines_of(const FoldView &v, const LineList &L, int n,
+                                                  int start) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int q = lane >> 3, sub = lane & 7;
   const uint4 *c4r = reinterpret_cast<const uint4 *>(v.cnt);
   uint4 *c4 = reinterpret_cast<uint4 *>(v.cnt);
+  uint4 *h4 = reinterpret_cast<uint4 *>(v.hit);
   float4 *o4 = reinterpret_cast<float4 *>(v.occ);
   uint32_t touched = 0;
   const int quads = (n + 3) >> 2;
@@ -283,9 +274,10 @@ __device__ __forceinline__ uint32_t fold_line_list(const FoldView &v, const uint
 #pragma unroll
     for (int u = 0; u < kQuads; ++u) {
       const int k = 4 * (i0 + u * warps) + q;
-      at[u] = k < n ? ((start + list[k]) << 3) + sub : -1;  // index of the 16-byte piece
+      // index of the 16-byte piece
+      at[u] = k < n ? ((start + L.line[kHot ? kListLines - 1 - k : k]) << 3) + sub : -1;
     }
-    uint4 c[kQuads];
+    uint4 c[kQuads], hc[kHot ? kQuads : 1];
     float4 o[kQuads];
 #pragma unroll
     for (int u = 0; u < kQuads; ++u)
@@ -293,22 +285,27 @@ __device__ __forceinline__ uint32_t fold_line_list(const FoldView &v, const uint
 #pragma unroll
     for (int u = 0; u < kQuads; ++u)
       if (at[u] >= 0) o[u] = o4[at[u]];
+    if constexpr (kHot) {
+#pragma unroll
+      for (int u = 0; u < kQuads; ++u)
+        if (at[u] >= 0) hc[u] = __ldcg(h4 + at[u]);
+    }
 #pragma unroll
     for (int u = 0; u < kQuads; ++u) {
       if (at[u] < 0 || !any_set(c[u])) continue;
-      const int h = at[u] << 2;
       const uint32_t cc[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
       float oo[4] = {o[u].x, o[u].y, o[u].z, o[u].w};
+      uint32_t hh[4] = {0u, 0u, 0u, 0u};
+      if constexpr (kHot) {
+        hh[0] = hc[u].x, hh[1] = hc[u].y, hh[2] = hc[u].z, hh[3] = hc[u].w;
+        if (any_set(hc[u])) h4[at[u]] = make_uint4(0u, 0u, 0u, 0u);
+      }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         touched += cc[e] != 0u;
-        if (cc[e] & kHitFlag) {  // rare: queued, or folded here with its hit count
-          oo[e] = fold_or_queue(v, hq, h + e, cc[e], oo[e]);
-        } else {
-          // no hit: the same arithmetic for every lane, kept where counted
-          const float f = fold_value(v, static_cast<int>(cc[e]), 0, oo[e]);
-          oo[e] = cc[e] ? f : oo[e];
-        }
+        // the same arithmetic for every lane, kept where counted
+        const float f = fold_value(v, static_cast<int>(cc[e] & kOpMask), static_cast<int>(hh[e]), oo[e]);
+        oo[e] = cc[e] ? f : oo[e];
       }
       o4[at[u]] = make_float4(oo[0], oo[1], oo[2], oo[3]);
       c4[at[u]] = make_uint4(0u, 0u, 0u, 0u);
@@ -317,17 +314,12 @@ __device__ __forceinline__ uint32_t fold_line_list(const FoldView &v, const uint
   return touched;
 }
 
-// Folds the queued hit voxels (after a CTA barrier that follows every
-// fold_line_list of the item) and empties the queue; ends with a CTA
-// barrier.  The stored value is read back: the list fold wrote it unchanged.
-__device__ __forceinline__ void fold_hit_queue(const FoldView &v, HitQueue &hq) {
-  const int n = min(hq.n, kHitCap);
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    const int h = hq.h[e];
-    v.occ[h] = fold_counter(v, h, hq.c[e], v.occ[h]);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) hq.n = 0;
+// Fold of the CTA's list: n.x lines without a hit, n.y with one.
+template <int kQuads, bool kL2>
+__device__ __forceinline__ uint32_t fold_line_list(const FoldView &v, const LineList &L, int2 n,
+                                                   int start) {
+  const uint32_t touched = fold_lines_of<kQuads, kL2, false>(v, L, n.x, start);
+  return touched + fold_lines_of<1, kL2, true>(v, L, n.y, start);
 }
 
 // The vnum % 4 voxels after the last whole group, one per thread 0..2.

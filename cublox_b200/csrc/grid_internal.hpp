@@ -22,6 +22,8 @@ struct FetchScratch {
   uint8_t *fstate = nullptr;
   int64_t fcap = 0;
 };
+// Bytes of one set of a map's line flags (16-byte loads start on its lines).
+inline size_t flag_bytes(int nlines) { return (static_cast<size_t>(nlines) + 255) & ~size_t(255); }
 }  // namespace cublox_b200
 
 struct cublox_grid {
@@ -77,7 +79,7 @@ struct cublox_grid {
   int lay_code = 0;     // brick sides as log2 digits x y z (320: 8 x 4 x 1)
   int64_t nalloc = 0;
   int nlines = 0;       // nalloc / 32
-  uint8_t *d_dirty = nullptr;  // line flags (kernels.cuh)
+  uint8_t *d_dirty = nullptr;  // line flags, then those of lines with a hit (kernels.cuh)
   int nbr[3] = {0, 0, 0};      // bricks per axis in the current layout
 
   float *d_occ = nullptr;

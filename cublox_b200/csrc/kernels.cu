@@ -50,8 +50,7 @@ __device__ __forceinline__ bool cast_one(const RayParams &p, float ex,
     atomicAdd(p.cnt + h, 1u);
     mark_line(p, h, last);
     if (!w.clipped) {
-      atomicOr(p.cnt + h, kHitFlag);
-      atomicAdd(p.hit + h, 1u);
+      mark_hit(p, h, 1u);
       ++h_incs;
     }
     ++incs;
@@ -165,7 +164,7 @@ __global__ void __launch_bounds__(256) fold_lines_kernel(const ApplyParams p) {
   const FoldView v = fold_view(p);
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  uint32_t touched = fold_lines<8, false>(v, p.dirty, warp * 32, p.nlines, warps * 32);
+  uint32_t touched = fold_lines<8, false>(v, p.dirty, p.hot, warp * 32, p.nlines, warps * 32);
   if (kStats) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
@@ -176,31 +175,18 @@ __global__ void __launch_bounds__(256) fold_lines_kernel(const ApplyParams p) {
 }
 
 // Fold of the flagged lines through per-CTA line lists (fold.cuh,
-// build_line_list / fold_line_list): CTA b takes items of kListLines lines
-// b, b + grid, ... and loads the next item's flags before folding the
-// current list.
+// build_line_list / fold_line_list), one item of lines per CTA.
 template <bool kStats>
 __global__ void __launch_bounds__(kListThreads, 4) fold_list_kernel(const ApplyParams p,
                                                                      int item_lines) {
   __shared__ LineList L;
-  __shared__ HitQueue hq;
-  if (threadIdx.x == 0) hq.n = 0;  // the first read follows build_line_list's barriers
   const FoldView v = fold_view(p);
-  const int items = (p.nlines + item_lines - 1) / item_lines;
-  auto count_of = [&](int it) { return min(item_lines, p.nlines - it * item_lines); };
-  int it = blockIdx.x;
-  uint4 f = make_uint4(0u, 0u, 0u, 0u);
-  if (it < items) f = load_line_flags(p.dirty, it * item_lines, count_of(it));
-  uint32_t touched = 0;
-  for (; it < items; it += gridDim.x) {
-    const int start = it * item_lines;
-    const int n = build_line_list(line_flag_bits(f), L, p.dirty, start, count_of(it));
-    const int next = it + gridDim.x;
-    if (next < items) f = load_line_flags(p.dirty, next * item_lines, count_of(next));
-    touched += fold_line_list<4, false>(v, L.line, n, start, &hq);
-    __syncthreads();
-    fold_hit_queue(v, hq);  // ends with a barrier: the list is rewritten next
-  }
+  const int start = blockIdx.x * item_lines;
+  const int count = min(item_lines, p.nlines - start);
+  const uint4 f = load_line_flags(p.dirty, start, count);
+  const uint4 fh = load_line_flags(p.hot, start, count);
+  const int2 n = build_line_list(line_flag_bits(f), line_flag_bits(fh), L, p.dirty, p.hot, start, count);
+  uint32_t touched = fold_line_list<3, false>(v, L, n, start);
   if (kStats) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
@@ -604,6 +590,10 @@ __global__ void __launch_bounds__(1024) viz_kernel(const VizParams p) {
   if (threadIdx.x == 0) *p.written = s_base < p.max_points ? s_base : p.max_points;
 }
 
+// Lines per item of the list fold: 512 and 2,048 fold a 262,144-ray scan in
+// 191 and 158 us, 1,024 in 154 (4,096, a CTA walking several: 211).
+constexpr int kPlainItemLines = 1024;
+
 int sm_count() {
   static int n = 0;
   if (n == 0) {
@@ -644,14 +634,14 @@ void launch_step_count(const RayParams &p, cudaStream_t s) {
 void launch_apply(const ApplyParams &p, cudaStream_t s) {
   if (p.variant == 2) {
     if (p.nlines <= 0) return;
-    // items of up to 4,096 lines, smaller for small maps so that every SM
-    // gets some (a multiple of 16 lines keeps the 16-byte flag loads aligned)
+    // items of up to kPlainItemLines lines, smaller for small maps so that
+    // every SM gets some (a multiple of 16 lines keeps the 16-byte flag
+    // loads aligned)
     const int cap = sm_count() * 4;
     int item_lines = (p.nlines + cap - 1) / cap;
     item_lines = ((item_lines + 255) / 256) * 256;
-    if (item_lines > kListLines) item_lines = kListLines;
-    int grid = (p.nlines + item_lines - 1) / item_lines;
-    if (grid > cap) grid = cap;
+    if (item_lines > kPlainItemLines) item_lines = kPlainItemLines;
+    const int grid = (p.nlines + item_lines - 1) / item_lines;
     if (p.stats)
       fold_list_kernel<true><<<grid, kListThreads, 0, s>>>(p, item_lines);
     else

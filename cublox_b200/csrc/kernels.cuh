@@ -8,6 +8,7 @@
 //   dirty  uint8[A/32]  per 32-voxel line of the arrays: 1 if the scan being
 //                     integrated has counted a voxel of the line; zero
 //                     between scans
+//   hot    uint8[A/32]  the same for lines in which it has counted a hit
 // A voxel's ring-buffer slot per axis is s = l + h (local index l in
 // [-h, h], utils.cuh:60-70), as in the reference's hash
 // ((sx*ny + sy)*nz + sz) (utils.cuh:131-136).
@@ -68,6 +69,7 @@ struct RayParams {
   uint32_t *err;
   VoxLayout lay;
   uint8_t *dirty;  // line flags to set, or null (the fold sweeps every line)
+  uint8_t *hot;    // flags of lines with a hit; null where dirty is
 };
 
 struct ApplyParams {
@@ -81,6 +83,7 @@ struct ApplyParams {
   int variant;                // 0 scalar sweep, 1 vector sweep, 2 flagged lines
                               // (per-CTA line lists), 3 flagged lines (per warp)
   uint8_t *dirty;             // variants 2, 3: line flags (cleared as folded)
+  uint8_t *hot;               // the same of lines with a hit
   int nlines;                 // variants 2, 3: lines
   uint32_t *err;              // error word (a bounded wait that gave up)
 };

@@ -147,7 +147,7 @@ int cublox_integrate_noalloc(const cublox_map_view *map, const float *xyz_soa, i
   p.lay.bs[0] = mapsz[1] * mapsz[2];
   p.lay.bs[1] = mapsz[2];
   p.lay.bs[2] = 1;
-  p.dirty = nullptr;
+  p.dirty = p.hot = nullptr;
 
   BinnedScratch b{reinterpret_cast<int *>(base), reinterpret_cast<int *>(base + kOffHist),
                   reinterpret_cast<int *>(base + kOffCursor),

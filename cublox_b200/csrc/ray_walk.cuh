@@ -112,6 +112,13 @@ __device__ __forceinline__ void mark_line(const RayParams &p, int h, int &last) 
   }
 }
 
+// Count a hit at address h (of a voxel whose line is flagged as counted).
+__device__ __forceinline__ void mark_hit(const RayParams &p, int h, uint32_t hits) {
+  atomicOr(p.cnt + h, kHitFlag);
+  atomicAdd(p.hit + h, hits);
+  if (p.hot) p.hot[h >> kLineShift] = 1;
+}
+
 // One step, tie rule of kernels.cu:120-136.  Returns the axis stepped.
 __device__ __forceinline__ int ray_step(RayWalk &w, const RayParams &p) {
   int a;

@@ -228,10 +228,8 @@ __global__ void __launch_bounds__(512, 1) walk_kernel(const RayParams p, const i
       }
       const uint32_t hkey = e_hit ? ekey : (kNoKey | lane);
       const uint32_t hp = __match_any_sync(0xffffffffu, hkey);
-      if (e_hit && lane == __ffs(hp) - 1) {
-        atomicOr(p.cnt + hkey, kHitFlag);
-        atomicAdd(p.hit + hkey, static_cast<uint32_t>(__popc(hp)));
-      }
+      if (e_hit && lane == __ffs(hp) - 1)
+        mark_hit(p, static_cast<int>(hkey), static_cast<uint32_t>(__popc(hp)));
     }
   }
   __syncthreads();
