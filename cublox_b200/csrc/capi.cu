@@ -1361,14 +1361,21 @@ static int ensure_fout(FetchScratch *sc, cudaStream_t st, int64_t n) {
   return CUBLOX_OK;
 }
 
-// Bytes of the query block for nq centres cut into nu work units (the
-// layout fetch_impl uses).
-static size_t fetch_query_bytes(int nq, int nu) {
-  auto al = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
-  const size_t ll = al(sizeof(long long) * std::max(nu, 1));
-  return al(sizeof(float) * 3 * nq) + al(sizeof(int) * 8 * nq) + al(sizeof(float) * nq) +
-         al(sizeof(int) * std::max(nu, 1)) + 4 * ll;
-}
+// The query block of a fetch in its scratch: queries | units | columns |
+// level masks | rows | kept | offsets.
+struct FetchBlock {
+  size_t units, col, mask, row, kept, offsets, bytes;
+  FetchBlock(size_t nq, size_t nu, size_t cols, size_t words, size_t rows) {
+    auto al = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
+    units = al(sizeof(FetchQuery) * nq);
+    col = units + al(sizeof(int2) * nu);
+    mask = col + al(sizeof(int) * cols);
+    row = mask + al(sizeof(uint32_t) * words);
+    kept = row + al(sizeof(int) * rows);
+    offsets = kept + al(sizeof(int) * nq);
+    bytes = offsets + al(sizeof(long long) * (nq + 1));
+  }
+};
 
 static int fetch_impl(cublox_grid *g, cudaStream_t st, const float *centers, int nq,
                       float radius, int filter, int max_results, int64_t *kept,
@@ -1382,62 +1389,64 @@ static int fetch_impl(cublox_grid *g, cudaStream_t st, const float *centers, int
     if (offsets) offsets[0] = 0;
     return CUBLOX_OK;
   }
-  std::vector<int> boxes(8 * static_cast<size_t>(nq));
-  std::vector<float> r2(nq);
-  std::vector<long long> cand(nq);
-  long long all_cand = 0;
-  for (int q = 0; q < nq; ++q) {
-    const QueryBox b = plan_query(g, centers + 3 * static_cast<size_t>(q), radius);
-    std::memcpy(&boxes[8 * static_cast<size_t>(q)], b.box, sizeof(b.box));
-    r2[q] = b.r2;
-    const long long nx = b.box[1] - b.box[0] + 1, ny = b.box[3] - b.box[2] + 1,
-                    nz = b.box[5] - b.box[4] + 1;
-    cand[q] = (nx > 0 && ny > 0 && nz > 0) ? nx * ny * nz : 0;
-    all_cand += cand[q];
-  }
-  // about 32 units per SM, never below kFetchMinUnit candidates
-  int sms = 148;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device) != cudaSuccess) {
-    cudaGetLastError();
-    sms = 148;
-  }
-  const long long unit = std::max<long long>(kFetchMinUnit, all_cand / (32LL * sms) + 1);
-  std::vector<int> uq;
-  std::vector<long long> ut0;
-  for (int q = 0; q < nq; ++q)
-    for (long long t = 0; t < cand[q]; t += unit) {
-      uq.push_back(q);
-      ut0.push_back(t);
+  FetchParams p{};
+  // tiles: the bricks' columns (at most 32, as in every layout of 32-voxel
+  // bricks); in the reference's order, 8 x 4 columns
+  p.lt[0] = g->lay_code == 0 ? 3 : g->lay.lb[0];
+  p.lt[1] = g->lay_code == 0 ? 2 : g->lay.lb[1];
+  std::vector<FetchQuery> queries(nq);
+  std::vector<int2> units;
+  int64_t cols = 0, words = 0, rows = 0;
+  int most = 1;
+  for (int i = 0; i < nq; ++i) {
+    const float *c = centers + 3 * static_cast<size_t>(i);
+    const QueryBox b = plan_query(g, c, radius);
+    FetchQuery &q = queries[i];
+    q = FetchQuery{};
+    for (int a = 0; a < 3; ++a) {
+      q.c[a] = c[a];
+      q.g0[a] = b.box[2 * a];
+      q.n[a] = b.box[2 * a + 1] - b.box[2 * a] + 1;
     }
-  const int nu = static_cast<int>(uq.size());
-  const size_t b_cent = sizeof(float) * 3 * nq, b_box = sizeof(int) * 8 * nq,
-               b_r2 = sizeof(float) * nq, b_uq = sizeof(int) * std::max(nu, 1),
-               b_ll = sizeof(long long) * std::max(nu, 1);
-  auto al = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
-  const size_t o_box = al(b_cent), o_r2 = o_box + al(b_box), o_uq = o_r2 + al(b_r2),
-               o_ut0 = o_uq + al(b_uq), o_cnt = o_ut0 + al(b_ll), o_off = o_cnt + al(b_ll),
-               o_lim = o_off + al(b_ll), total = o_lim + al(b_ll);
-  int rc = ensure_fq(sc, st, total);
+    q.r2 = b.r2;
+    q.row0 = rows;
+    q.col0 = cols;
+    q.mask0 = words;
+    if (q.n[0] <= 0 || q.n[1] <= 0 || q.n[2] <= 0) {
+      q.n[0] = q.n[1] = q.n[2] = 0;
+      continue;
+    }
+    for (int a = 0; a < 2; ++a) {
+      const int m = g->map[a], h = g->half[a], tiles = (m + (1 << p.lt[a]) - 1) >> p.lt[a];
+      const int first = global_to_local(q.g0[a], m, h) + h;
+      const int last = global_to_local(q.g0[a] + q.n[a] - 1, m, h) + h;
+      q.t0[a] = first >> p.lt[a];
+      // around the ring where the box wraps; its two ends may share a tile
+      const int span = (last >> p.lt[a]) - q.t0[a] + 1 + (last < first ? tiles : 0);
+      q.nt[a] = std::min(span, tiles);
+    }
+    for (int t = 0; t < q.nt[0]; ++t) units.push_back(make_int2(i, t));
+    most = std::max(most, q.nt[1]);
+    rows += q.n[0];
+    cols += static_cast<int64_t>(q.n[0]) * q.n[1];
+    if (filter >= 0) words += static_cast<int64_t>(q.n[0]) * q.n[1] * ((q.n[2] + 31) / 32);
+  }
+  const int nu = static_cast<int>(units.size());
+  const FetchBlock blk(static_cast<size_t>(nq), units.size(), static_cast<size_t>(cols),
+                       static_cast<size_t>(words), static_cast<size_t>(rows));
+  int rc = ensure_fq(sc, st, blk.bytes);
   if (rc) return rc;
   char *base = static_cast<char *>(sc->fq);
-  CK(cudaMemcpyAsync(base, centers, b_cent, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(base + o_box, boxes.data(), b_box, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(base + o_r2, r2.data(), b_r2, cudaMemcpyHostToDevice, st));
-  if (nu > 0) {
-    CK(cudaMemcpyAsync(base + o_uq, uq.data(), sizeof(int) * nu, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(base + o_ut0, ut0.data(), sizeof(long long) * nu, cudaMemcpyHostToDevice,
+  CK(cudaMemcpyAsync(base, queries.data(), sizeof(FetchQuery) * nq, cudaMemcpyHostToDevice, st));
+  if (nu > 0)
+    CK(cudaMemcpyAsync(base + blk.units, units.data(), sizeof(int2) * nu, cudaMemcpyHostToDevice,
                        st));
-  }
-  FetchParams p{};
   p.occ = g->d_occ;
-  p.centers = reinterpret_cast<const float *>(base);
-  p.qbox = reinterpret_cast<const int *>(base + o_box);
-  p.qr2 = reinterpret_cast<const float *>(base + o_r2);
+  p.queries = reinterpret_cast<const FetchQuery *>(base);
   p.nq = nq;
-  p.uq = reinterpret_cast<const int *>(base + o_uq);
-  p.ut0 = reinterpret_cast<const long long *>(base + o_ut0);
+  p.units = reinterpret_cast<const int2 *>(base + blk.units);
   p.nu = nu;
-  p.unit = unit;
+  p.most_tiles = most;
   for (int a = 0; a < 3; ++a) {
     p.win[a] = g->origin_i[a];
     p.half[a] = g->half[a];
@@ -1450,65 +1459,58 @@ static int fetch_impl(cublox_grid *g, cudaStream_t st, const float *centers, int
   p.l_occ = g->l_occ;
   p.l_unknown = g->l_unknown;
   p.filter = filter;
+  p.cap = max_results > 0 ? max_results : 500000;  // OccupancyGrid.cpp:292
   p.lay = g->lay;
-  p.counts = reinterpret_cast<long long *>(base + o_cnt);
-  p.offsets = reinterpret_cast<const long long *>(base + o_off);
-  p.limits = reinterpret_cast<const long long *>(base + o_lim);
-  p.err = g->d_err;
-  launch_fetch(p, 1, st);
+  p.col = reinterpret_cast<int *>(base + blk.col);
+  p.mask = write && filter >= 0 ? reinterpret_cast<uint32_t *>(base + blk.mask) : nullptr;
+  p.row = reinterpret_cast<int *>(base + blk.row);
+  p.kept = reinterpret_cast<int *>(base + blk.kept);
+  p.offsets = reinterpret_cast<long long *>(base + blk.offsets);
+  launch_fetch_count(p, st);
   CK_LAUNCH();
-  std::vector<long long> ucnt(std::max(nu, 1)), uoff(std::max(nu, 1)), ulim(std::max(nu, 1));
-  if (nu > 0) {
-    CK(cudaMemcpyAsync(ucnt.data(), p.counts, sizeof(long long) * nu, cudaMemcpyDeviceToHost,
-                       st));
-    CK(cudaStreamSynchronize(st));
-  }
-  // Per query, its units in order: each keeps what fits under the cap, and
-  // writes after everything its query kept before it.
-  const long long cap_q = max_results > 0 ? max_results : 500000;  // OccupancyGrid.cpp:292
-  std::vector<long long> off(nq + 1);
-  off[0] = 0;
-  for (int u = 0, q = 0; q < nq; ++q) {
-    long long running = 0;
-    for (; u < nu && uq[u] == q; ++u) {
-      uoff[u] = off[q] + std::min(running, cap_q);
-      ulim[u] = std::max(0LL, std::min(ucnt[u], cap_q - running));
-      running += ucnt[u];
-    }
-    const long long lim = std::min(running, cap_q);
-    off[q + 1] = off[q] + lim;
-    if (kept) kept[q] = lim;
-  }
-  if (offsets)
-    for (int q = 0; q <= nq; ++q) offsets[q] = off[q];
-  if (!write) return CUBLOX_OK;
-  const long long total_s = off[nq];
-  if (vpos && vstate) {
-    vpos->resize(3 * static_cast<size_t>(total_s));
-    vstate->resize(static_cast<size_t>(total_s));
-    out_pos = vpos->data();
-    out_state = vstate->data();
-    capacity = total_s;
-  }
-  if (total_s > capacity)
-    return fail(CUBLOX_ERR_INVALID, "fetch: output capacity " + std::to_string(capacity) +
-                                        " < " + std::to_string(total_s) + " samples");
-  if (total_s == 0) return CUBLOX_OK;
-  rc = ensure_fout(sc, st, total_s);
-  if (rc) return rc;
-  CK(cudaMemcpyAsync(base + o_off, uoff.data(), sizeof(long long) * nu, cudaMemcpyHostToDevice,
-                     st));
-  CK(cudaMemcpyAsync(base + o_lim, ulim.data(), sizeof(long long) * nu, cudaMemcpyHostToDevice,
-                     st));
+  // The samples are written without waiting for their number where the
+  // outputs of earlier fetches have room for them.
+  p.room = sc->fcap;
   p.out_pos = sc->fpos;
   p.out_state = sc->fstate;
-  launch_fetch(p, 2, st);
-  CK_LAUNCH();
+  if (write && p.room > 0) {
+    launch_fetch_write(p, st);
+    CK_LAUNCH();
+  }
+  std::vector<long long> off(nq + 1);
+  CK(cudaMemcpyAsync(off.data(), p.offsets, sizeof(long long) * (nq + 1), cudaMemcpyDeviceToHost,
+                     st));
+  CK(cudaStreamSynchronize(st));
+  for (int i = 0; i < nq; ++i)
+    if (kept) kept[i] = off[i + 1] - off[i];
+  if (offsets)
+    for (int i = 0; i <= nq; ++i) offsets[i] = off[i];
+  if (!write) return CUBLOX_OK;
+  const long long total = off[nq];
+  if (vpos && vstate) {
+    vpos->resize(3 * static_cast<size_t>(total));
+    vstate->resize(static_cast<size_t>(total));
+    out_pos = vpos->data();
+    out_state = vstate->data();
+    capacity = total;
+  }
+  if (total > capacity)
+    return fail(CUBLOX_ERR_INVALID, "fetch: output capacity " + std::to_string(capacity) +
+                                        " < " + std::to_string(total) + " samples");
+  if (total == 0) return CUBLOX_OK;
+  if (total > p.room) {
+    if ((rc = ensure_fout(sc, st, total))) return rc;
+    p.room = sc->fcap;
+    p.out_pos = sc->fpos;
+    p.out_state = sc->fstate;
+    launch_fetch_write(p, st);
+    CK_LAUNCH();
+  }
   if (out_pos)
-    CK(cudaMemcpyAsync(out_pos, sc->fpos, sizeof(float) * 3 * static_cast<size_t>(total_s),
+    CK(cudaMemcpyAsync(out_pos, sc->fpos, sizeof(float) * 3 * static_cast<size_t>(total),
                        cudaMemcpyDeviceToHost, st));
   if (out_state)
-    CK(cudaMemcpyAsync(out_state, sc->fstate, static_cast<size_t>(total_s),
+    CK(cudaMemcpyAsync(out_state, sc->fstate, static_cast<size_t>(total),
                        cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   return CUBLOX_OK;
@@ -1525,10 +1527,15 @@ int cublox_b200::detail::fetch_into(cublox_grid *g, cudaStream_t st, const float
                     nullptr, nullptr, 0, true, &pos, &state, sc);
 }
 
+size_t cublox_b200::detail::fetch_block_bytes(int centres) {
+  // boxes of 48 x 48 columns (2 m at 0.1 m), overlapping 7 tiles along x
+  const size_t n = static_cast<size_t>(std::max(centres, 0));
+  return FetchBlock(n, 7 * n, 48 * 48 * n, 2 * 48 * 48 * n, 48 * n).bytes;
+}
+
 int cublox_b200::detail::reserve_fetch(FetchScratch *sc, int centres, int64_t samples,
                                        cudaStream_t st) {
-  // work units: at most 32 per SM plus one per centre (fetch_impl's cut)
-  int rc = ensure_fq(sc, st, fetch_query_bytes(centres, centres + 32 * 160));
+  int rc = ensure_fq(sc, st, fetch_block_bytes(centres));
   if (rc) return rc;
   return ensure_fout(sc, st, samples);
 }

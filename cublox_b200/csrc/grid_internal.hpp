@@ -11,9 +11,8 @@
 #include "kernels.cuh"
 
 namespace cublox_b200 {
-// Device scratch of a sphere fetch: the query block (centres | boxes |
-// radii | work units | per-unit counts, offsets and limits) and the sample
-// outputs.  A grid grows its own on demand; the server owns one, sized when
+// Device scratch of a sphere fetch: the query block (queries | work units |
+// columns | rows | samples per query | offsets) and the sample outputs.  A grid grows its own on demand; the server owns one, sized when
 // it is created, shared by its fetches (they run one at a time).
 struct FetchScratch {
   void *fq = nullptr;
@@ -193,6 +192,9 @@ int fetch_into(cublox_grid *g, cudaStream_t st, const float *centers, int nq, fl
                int filter, int max_results, std::vector<int64_t> &offsets,
                std::vector<float> &pos, std::vector<uint8_t> &state,
                FetchScratch *sc = nullptr);
+// Device bytes of the query block of a fetch of that many centres (of up to 2
+// m at 0.1 m; larger boxes grow it).
+size_t fetch_block_bytes(int centres);
 // Size `sc` for fetches of up to `centres` centres and `samples` samples, so
 // that such fetches allocate nothing.
 int reserve_fetch(FetchScratch *sc, int centres, int64_t samples, cudaStream_t st);

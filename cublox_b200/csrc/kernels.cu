@@ -323,89 +323,6 @@ __global__ void __launch_bounds__(256) relayout_kernel(const float *src, float *
   }
 }
 
-// Sphere fetch over host-clipped candidate boxes, one block per query
-// (grid-stride), candidates in (x, y, z) order with z fastest so that
-// consecutive threads read consecutive voxels of one column.  Pass 1 counts,
-// pass 2 writes the first `limits[q]` samples at `offsets[q]` in that order.
-template <int kPass>
-__global__ void __launch_bounds__(256) fetch_kernel(const FetchParams p) {
-  __shared__ int warp_tot[8];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int u = blockIdx.x; u < p.nu; u += gridDim.x) {
-    const int q = p.uq[u];
-    const int *b = p.qbox + 8 * q;
-    const int gx0 = b[0], gy0 = b[2], gz0 = b[4];
-    const int nx = b[1] - b[0] + 1, nyy = b[3] - b[2] + 1, nzz = b[5] - b[4] + 1;
-    const float c[3] = {p.centers[3 * q], p.centers[3 * q + 1],
-                        p.centers[3 * q + 2]};
-    const float r2 = p.qr2[q];
-    long long running = 0;
-    const long long limit = kPass == 2 ? p.limits[u] : 0;
-    const long long base_off = kPass == 2 ? p.offsets[u] : 0;
-    const long long all = (nx > 0 && nyy > 0 && nzz > 0)
-                              ? static_cast<long long>(nx) * nyy * nzz
-                              : 0;
-    const long long t_begin = p.ut0[u];
-    const long long total = min(all, t_begin + p.unit);  // end of this unit
-    for (long long t0 = t_begin; t0 < total; t0 += blockDim.x) {
-      if (kPass == 2 && running >= limit) break;
-      const long long t = t0 + threadIdx.x;
-      bool keep = false;
-      float pos[3];
-      uint8_t state = 0;
-      if (t < total) {
-        const int iz = static_cast<int>(t % nzz);
-        const long long r = t / nzz;
-        const int iy = static_cast<int>(r % nyy);
-        const int ix = static_cast<int>(r / nyy);
-        const int g[3] = {gx0 + ix, gy0 + iy, gz0 + iz};
-        float d[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const float tt = p.ctr ? static_cast<float>(g[a])
-                                 : fadd(static_cast<float>(g[a]), 0.5f);
-          pos[a] = fmul(tt, p.res);
-          d[a] = (p.fp & kFpFetchDFma) ? ffma(tt, p.res, -c[a])
-                                       : fsub(pos[a], c[a]);
-        }
-        const float s = sos(d[0], d[1], d[2], (p.fp >> kFpFetchSosShift) & 7u);
-        if (!(s > r2)) {
-          const int h = vox_addr(p.lay, global_to_local(g[0], p.map[0], p.half[0]) + p.half[0],
-                                 global_to_local(g[1], p.map[1], p.half[1]) + p.half[1],
-                                 global_to_local(g[2], p.map[2], p.half[2]) + p.half[2]);
-          const float l = fadd(p.occ[h], p.l_unknown);
-          state = l >= p.l_occ ? 2 : (l < p.l_free ? 1 : 0);
-          keep = p.filter < 0 || static_cast<int>(state) == p.filter;
-        }
-      }
-      const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-      if (lane == 0) warp_tot[warp] = __popc(bal);
-      __syncthreads();
-      int before = 0, blk = 0;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        const int v = warp_tot[w];
-        before += w < warp ? v : 0;
-        blk += v;
-      }
-      if (kPass == 2 && keep) {
-        const long long rank =
-            running + before + __popc(bal & ((1u << lane) - 1u));
-        if (rank < limit) {
-          const long long o = base_off + rank;
-          p.out_pos[3 * o + 0] = pos[0];
-          p.out_pos[3 * o + 1] = pos[1];
-          p.out_pos[3 * o + 2] = pos[2];
-          p.out_state[o] = state;
-        }
-      }
-      running += blk;
-      __syncthreads();
-    }
-    if (kPass == 1 && threadIdx.x == 0) p.counts[u] = running;
-  }
-}
-
 // Host-side float->int of the reference's point queries (x86 cvttss2si:
 // NaN or out of range gives INT_MIN).
 __device__ __forceinline__ int f2i_hostlike(float v) {
@@ -704,17 +621,6 @@ void launch_clear(const ClearParams &p, cudaStream_t s) {
   const size_t smem = sizeof(uint32_t) * wy + sizeof(int) * (p.map[2] + 1);
   int grid = p.map[0];
   clear_kernel<<<grid, 256, smem, s>>>(p);
-}
-
-void launch_fetch(const FetchParams &p, int pass, cudaStream_t s) {
-  if (p.nu <= 0) return;
-  int grid = p.nu;
-  const int cap = sm_count() * 8;
-  if (grid > cap) grid = cap;
-  if (pass == 1)
-    fetch_kernel<1><<<grid, 256, 0, s>>>(p);
-  else
-    fetch_kernel<2><<<grid, 256, 0, s>>>(p);
 }
 
 void launch_query(const QueryParams &p, cudaStream_t s) {

@@ -103,34 +103,41 @@ struct ClearParams {
   int nbr[3];        // bricks per axis
 };
 
-// A fetch's candidates are cut into work units of `unit` consecutive
-// candidates of one query (in the query's (x, y, z) order), so that one
-// large sphere spreads over the whole GPU while many small ones stay whole.
-constexpr int kFetchMinUnit = 8192;
+// One sphere of a fetch: its centre, squared radius and candidate box, and
+// the tiles (of 2^lt[0] x 2^lt[1] slots) that the box overlaps.
+struct FetchQuery {
+  float c[3], r2;
+  int g0[3], n[3];  // first global index and extent per axis (0: empty)
+  int t0[2], nt[2]; // first tile and tiles (around the ring) along x and y
+  long long row0;   // the query's first row in FetchParams::row
+  long long col0;   // and column in FetchParams::col
+  long long mask0;  // and word in FetchParams::mask
+};
 
 struct FetchParams {
   const float *occ;
-  const float *centers;  // 3 per query
-  const int *qbox;       // 8 ints per query: gx0 gx1 gy0 gy1 gz0 gz1 pad pad
-  const float *qr2;      // radius_sq per query
+  const FetchQuery *queries;
   int nq;
-  const int *uq;             // per unit: its query
-  const long long *ut0;      // per unit: its first candidate
+  const int2 *units;  // a query and a tile along x, within the query's
   int nu;
-  long long unit;            // candidates per unit
+  int most_tiles;     // along y, of any query
+  int lt[2];          // log2 of a tile's sides (columns), at most 32 columns
   int win[3], half[3], map[3];
   float res;
   int ctr;
   unsigned fp;
   float l_free, l_occ, l_unknown;
   int filter;
+  int cap;            // samples a query keeps at most
   VoxLayout lay;
-  long long *counts;         // pass 1 output: samples per unit
-  const long long *offsets;  // pass 2 input: where each unit's samples go
-  const long long *limits;   // pass 2: samples each unit keeps (the cap)
+  int *col;           // per column: samples before it in its row
+  uint32_t *mask;     // one state wanted: per column, a bit per level kept; else null
+  int *row;           // per row: samples before it in its query
+  int *kept;          // per query: samples it keeps
+  long long *offsets; // per query: where its samples go; [nq]: samples in all
+  long long room;     // samples the outputs hold; more are not written
   float *out_pos;
   uint8_t *out_state;
-  uint32_t *err;
 };
 
 struct QueryParams {
@@ -194,7 +201,9 @@ int kernel_binary_version();
 void launch_step_count(const RayParams &p, cudaStream_t s);
 void launch_apply(const ApplyParams &p, cudaStream_t s);
 void launch_clear(const ClearParams &p, cudaStream_t s);
-void launch_fetch(const FetchParams &p, int pass, cudaStream_t s);
+// Sphere fetch (fetch.cu): where each sample goes, then the samples.
+void launch_fetch_count(const FetchParams &p, cudaStream_t s);
+void launch_fetch_write(const FetchParams &p, cudaStream_t s);
 void launch_query(const QueryParams &p, cudaStream_t s);
 // Sensor-frame cloud -> world-frame SoA (the reference driver's
 // buildCloudInOdomFrame, src/main.cpp:640-693): non-finite points and points

@@ -231,10 +231,8 @@ void finish(cublox_server *s, Request *r, int error, const std::string &msg) {
 // Fetch scratch sized for cfg's fetch limits (the query block, 13 B a
 // sample).
 size_t fetch_scratch_bytes(const cublox_server_config &cfg) {
-  const size_t nq = static_cast<size_t>(cfg.max_fetch_centres);
-  const size_t nu = nq + 32 * 160;
-  return 4 * nq * 12 + 4 * nu * 40 + 13 * static_cast<size_t>(cfg.max_fetch_samples) +
-         (size_t(16) << 10);
+  return cublox_b200::detail::fetch_block_bytes(cfg.max_fetch_centres) +
+         13 * static_cast<size_t>(cfg.max_fetch_samples) + (size_t(16) << 10);
 }
 
 size_t scratch_bytes(const cublox_server_config &cfg) {
