@@ -106,6 +106,9 @@ def lib():
                                    i64], ctypes.c_int),
             "cublox_grid_fetch_batch": ([G, f, ctypes.c_int, ctypes.c_float, ctypes.c_int, ctypes.c_int, i64,
                                          f, u8, ctypes.c_int64], ctypes.c_int),
+            "cublox_grid_fetch_begin": ([G, f, ctypes.c_int, ctypes.c_float, ctypes.c_int, ctypes.c_int, i64],
+                                        ctypes.c_int),
+            "cublox_grid_fetch_read": ([G, f, u8, ctypes.c_int64], ctypes.c_int),
             "cublox_grid_fetch_counts": ([G, f, ctypes.c_int, ctypes.c_float, ctypes.c_int, ctypes.c_int,
                                           i64], ctypes.c_int),
             "cublox_grid_query_states": ([G, f, ctypes.c_int, u8], ctypes.c_int),
@@ -335,39 +338,29 @@ class OccupancyGrid:
 
         Returns (positions (n, 3) float32, states (n,) uint8), ordered by
         ascending (x, y, z) global voxel index."""
-        flt = -1 if state_filter is None else int(state_filter)
-        c = _f3(center)
-        counts = np.zeros(1, dtype=np.int64)
-        _check(lib().cublox_grid_fetch_counts(self._h, c, 1, float(radius), flt, int(max_results),
-                                              counts.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))),
-               "fetchOccupancyAround")
-        n = int(counts[0])
-        pos = np.empty((max(n, 1), 3), dtype=np.float32)
-        st = np.empty(max(n, 1), dtype=np.uint8)
-        got = ctypes.c_int64(0)
-        _check(lib().cublox_grid_fetch(self._h, c, float(radius), flt, int(max_results), _fp(pos),
-                                       st.ctypes.data_as(ctypes.POINTER(ctypes.c_uint8)), n,
-                                       ctypes.byref(got)), "fetchOccupancyAround")
-        return pos[: got.value], st[: got.value]
+        _, pos, st = self._fetch([center], radius, state_filter, max_results, "fetchOccupancyAround")
+        return pos, st
 
     def fetch_batch(self, centers, radius: float, state_filter=None, max_results: int = 0):
         """All centres in one launch: (offsets (n+1,), positions, states)."""
+        return self._fetch(centers, radius, state_filter, max_results, "fetch_batch")
+
+    def _fetch(self, centers, radius, state_filter, max_results, what):
         flt = -1 if state_filter is None else int(state_filter)
         c = np.ascontiguousarray(np.asarray(centers, dtype=np.float32).reshape(-1, 3))
         nq = c.shape[0]
-        counts = np.zeros(max(nq, 1), dtype=np.int64)
-        _check(lib().cublox_grid_fetch_counts(self._h, _fp(c), nq, float(radius), flt, int(max_results),
-                                              counts.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))),
-               "fetch_batch")
-        total = int(counts[:nq].sum())
         off = np.zeros(nq + 1, dtype=np.int64)
-        pos = np.empty((max(total, 1), 3), dtype=np.float32)
-        st = np.empty(max(total, 1), dtype=np.uint8)
-        _check(lib().cublox_grid_fetch_batch(self._h, _fp(c), nq, float(radius), flt, int(max_results),
-                                             off.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)), _fp(pos),
-                                             st.ctypes.data_as(ctypes.POINTER(ctypes.c_uint8)), total),
-               "fetch_batch")
-        return off, pos[:total], st[:total]
+        _check(lib().cublox_grid_fetch_begin(self._h, _fp(c), nq, float(radius), flt, int(max_results),
+                                             off.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))),
+               what)
+        total = int(off[nq])
+        pos = np.empty((total, 3), dtype=np.float32)
+        st = np.empty(total, dtype=np.uint8)
+        if total:
+            _check(lib().cublox_grid_fetch_read(self._h, _fp(pos),
+                                                st.ctypes.data_as(ctypes.POINTER(ctypes.c_uint8)), total),
+                   what)
+        return off, pos, st
 
     def fetch_viz(self, center, radius: float, state_filter=None, max_results: int = 0,
                   subsample_step: int = 1, max_viz_radius: float = 25.0, max_points: int = 200000,

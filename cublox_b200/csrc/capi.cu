@@ -12,7 +12,11 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <functional>
 #include <string>
+#include <system_error>
+#include <thread>
+#include <utility>
 #include <vector>
 
 #include "../../include/cublox_b200.h"
@@ -176,6 +180,7 @@ static void free_all(cublox_grid *g) {
   cublox_b200::detail::dfree(g->d_err);
   cublox_b200::detail::dfree(g->d_masks);
   if (g->h_masks) cublox_b200::detail::hfree(g->h_masks);
+  cublox_b200::detail::hfree(g->h_query);
   for (cudaEvent_t e : g->mask_ev)
     if (e) cudaEventDestroy(e);
   cublox_b200::detail::dfree(g->d_cloud);
@@ -1377,16 +1382,36 @@ struct FetchBlock {
   }
 };
 
-static int fetch_impl(cublox_grid *g, cudaStream_t st, const float *centers, int nq,
-                      float radius, int filter, int max_results, int64_t *kept,
-                      int64_t *offsets, float *out_pos, uint8_t *out_state, int64_t capacity,
-                      bool write, std::vector<float> *vpos = nullptr,
-                      std::vector<uint8_t> *vstate = nullptr, FetchScratch *sc = nullptr) {
+// Pinned host memory of a fetch scratch, grown geometrically.
+static int ensure_pinned(void **p, size_t *have, size_t bytes) {
+  if (bytes <= *have) return CUBLOX_OK;
+  bytes = std::max({bytes, 2 * *have, static_cast<size_t>(16) << 10});
+  cublox_b200::detail::hfree(*p);
+  *p = nullptr;
+  *have = 0;
+  if (cublox_b200::detail::hmalloc(p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(CUBLOX_ERR_NOMEM, "fetch: pinned allocation failed");
+  }
+  *have = bytes;
+  return CUBLOX_OK;
+}
+
+// Finds the fetch's samples: sc->hoff[0 .. nq] are the queries' offsets, and,
+// with `write`, the samples are in sc->fpos and sc->fstate when it returns.
+static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int nq, float radius,
+                     int filter, int max_results, bool write, FetchScratch *sc) {
   if (!g || (nq > 0 && !centers)) return fail(CUBLOX_ERR_INVALID, "fetch: null argument");
   if (!sc) sc = &g->fs;
   if (filter < -1 || filter > 2) return fail(CUBLOX_ERR_INVALID, "fetch: bad filter");
-  if (nq <= 0) {
-    if (offsets) offsets[0] = 0;
+  sc->pending = -1;
+  nq = std::max(nq, 0);
+  int rc = ensure_pinned(&sc->hoff, &sc->hoff_bytes, sizeof(long long) * (static_cast<size_t>(nq) + 1));
+  if (rc) return rc;
+  long long *off = static_cast<long long *>(sc->hoff);
+  off[0] = 0;
+  if (nq == 0) {
+    sc->pending = 0;
     return CUBLOX_OK;
   }
   FetchParams p{};
@@ -1434,8 +1459,7 @@ static int fetch_impl(cublox_grid *g, cudaStream_t st, const float *centers, int
   const int nu = static_cast<int>(units.size());
   const FetchBlock blk(static_cast<size_t>(nq), units.size(), static_cast<size_t>(cols),
                        static_cast<size_t>(words), static_cast<size_t>(rows));
-  int rc = ensure_fq(sc, st, blk.bytes);
-  if (rc) return rc;
+  if ((rc = ensure_fq(sc, st, blk.bytes))) return rc;
   char *base = static_cast<char *>(sc->fq);
   CK(cudaMemcpyAsync(base, queries.data(), sizeof(FetchQuery) * nq, cudaMemcpyHostToDevice, st));
   if (nu > 0)
@@ -1477,27 +1501,11 @@ static int fetch_impl(cublox_grid *g, cudaStream_t st, const float *centers, int
     launch_fetch_write(p, st);
     CK_LAUNCH();
   }
-  std::vector<long long> off(nq + 1);
-  CK(cudaMemcpyAsync(off.data(), p.offsets, sizeof(long long) * (nq + 1), cudaMemcpyDeviceToHost,
-                     st));
+  CK(cudaMemcpyAsync(off, p.offsets, sizeof(long long) * (static_cast<size_t>(nq) + 1),
+                     cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  for (int i = 0; i < nq; ++i)
-    if (kept) kept[i] = off[i + 1] - off[i];
-  if (offsets)
-    for (int i = 0; i <= nq; ++i) offsets[i] = off[i];
   if (!write) return CUBLOX_OK;
   const long long total = off[nq];
-  if (vpos && vstate) {
-    vpos->resize(3 * static_cast<size_t>(total));
-    vstate->resize(static_cast<size_t>(total));
-    out_pos = vpos->data();
-    out_state = vstate->data();
-    capacity = total;
-  }
-  if (total > capacity)
-    return fail(CUBLOX_ERR_INVALID, "fetch: output capacity " + std::to_string(capacity) +
-                                        " < " + std::to_string(total) + " samples");
-  if (total == 0) return CUBLOX_OK;
   if (total > p.room) {
     if ((rc = ensure_fout(sc, st, total))) return rc;
     p.room = sc->fcap;
@@ -1505,26 +1513,116 @@ static int fetch_impl(cublox_grid *g, cudaStream_t st, const float *centers, int
     p.out_state = sc->fstate;
     launch_fetch_write(p, st);
     CK_LAUNCH();
+    CK(cudaStreamSynchronize(st));
   }
-  if (out_pos)
-    CK(cudaMemcpyAsync(out_pos, sc->fpos, sizeof(float) * 3 * static_cast<size_t>(total),
-                       cudaMemcpyDeviceToHost, st));
-  if (out_state)
-    CK(cudaMemcpyAsync(out_state, sc->fstate, static_cast<size_t>(total),
-                       cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  sc->pending = total;
   return CUBLOX_OK;
+}
+
+// Device to pageable host memory.  From kThreadedCopy on, through the
+// scratch's pinned buffer in pieces that several threads take in turn, each
+// waiting for its piece's DMA and then copying it out, so that the copies
+// (and the first touch of the caller's fresh pages, which costs more than
+// they do) run side by side and beside the DMA: 54 MB into new arrays 3.4 ms,
+// against 10.9 ms by the runtime's own staging; 1.6 MB takes that 0.14 ms,
+// threads 0.12 to 0.28.
+static int copy_out(cublox_grid *g, cudaStream_t st, FetchScratch *sc,
+                    const std::pair<const void *, void *> *parts, const size_t *bytes, int n_parts) {
+  constexpr size_t kThreadedCopy = static_cast<size_t>(4) << 20;
+  constexpr size_t kPiece = static_cast<size_t>(512) << 10;
+  constexpr int kMostThreads = 8;
+  size_t all = 0;
+  for (int i = 0; i < n_parts; ++i)
+    if (parts[i].second) all += bytes[i];
+  if (all < kThreadedCopy) {
+    for (int i = 0; i < n_parts; ++i)
+      if (parts[i].second)
+        CK(cudaMemcpyAsync(parts[i].second, parts[i].first, bytes[i], cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    return CUBLOX_OK;
+  }
+  struct Piece {
+    const char *src;
+    char *dst;
+    size_t bytes;
+  };
+  std::vector<Piece> pieces;
+  for (int i = 0; i < n_parts; ++i)
+    for (size_t o = 0; parts[i].second && o < bytes[i]; o += kPiece)
+      pieces.push_back({static_cast<const char *>(parts[i].first) + o,
+                        static_cast<char *>(parts[i].second) + o, std::min(kPiece, bytes[i] - o)});
+  int rc;
+  const int cores = static_cast<int>(std::thread::hardware_concurrency());
+  const int threads = std::max(1, std::min(kMostThreads, cores / 2));
+  if ((rc = ensure_pinned(&sc->hcopy, &sc->hcopy_bytes, kPiece * threads))) return rc;
+  std::atomic<size_t> next{0};
+  std::atomic<int> error{cudaSuccess};
+  auto work = [&](int t) {
+    cudaEvent_t ev = nullptr;
+    cudaError_t e = cudaSetDevice(g->device);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    char *h = static_cast<char *>(sc->hcopy) + kPiece * t;
+    for (size_t i; e == cudaSuccess && (i = next.fetch_add(1)) < pieces.size();) {
+      const Piece &p = pieces[i];
+      if ((e = cudaMemcpyAsync(h, p.src, p.bytes, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
+          (e = cudaEventRecord(ev, st)) == cudaSuccess &&
+          (e = cudaEventSynchronize(ev)) == cudaSuccess)
+        std::memcpy(p.dst, h, p.bytes);
+    }
+    if (ev) cudaEventDestroy(ev);
+    if (e != cudaSuccess) error = e;
+  };
+  std::vector<std::thread> helpers;
+  int prev = -1;
+  if (cudaGetDevice(&prev) != cudaSuccess) cudaGetLastError();
+  try {
+    for (int t = 1; t < threads; ++t) helpers.emplace_back(work, t);
+  } catch (const std::system_error &) {  // no more threads: those there are do the work
+  }
+  work(0);
+  for (std::thread &h : helpers) h.join();
+  if (prev >= 0 && prev != g->device) cudaSetDevice(prev);
+  CK(static_cast<cudaError_t>(error.load()));
+  return CUBLOX_OK;
+}
+
+// The pending fetch's samples to host memory (null: not wanted).
+static int fetch_copy(cublox_grid *g, cudaStream_t st, FetchScratch *sc, float *out_pos,
+                      uint8_t *out_state) {
+  const size_t n = static_cast<size_t>(sc->pending);
+  if (n == 0) return CUBLOX_OK;
+  std::pair<const void *, void *> parts[2] = {{sc->fpos, out_pos}, {sc->fstate, out_state}};
+  size_t bytes[2] = {12 * n, n};
+  bool direct = false;  // pinned: the DMA's own destination
+  for (int i = 0; i < 2; ++i) {
+    if (!parts[i].second || mem_kind(parts[i].second) == 0) continue;
+    CK(cudaMemcpyAsync(parts[i].second, parts[i].first, bytes[i], cudaMemcpyDeviceToHost, st));
+    parts[i].second = nullptr;
+    direct = true;
+  }
+  if (direct) CK(cudaStreamSynchronize(st));
+  return copy_out(g, st, sc, parts, bytes, 2);
 }
 
 }  // extern "C"
 
 int cublox_b200::detail::fetch_into(cublox_grid *g, cudaStream_t st, const float *centers,
                                     int nq, float radius, int filter, int max_results,
-                                    std::vector<int64_t> &offsets, std::vector<float> &pos,
-                                    std::vector<uint8_t> &state, FetchScratch *sc) {
-  offsets.assign(static_cast<size_t>(nq) + 1, 0);
-  return fetch_impl(g, st, centers, nq, radius, filter, max_results, nullptr, offsets.data(),
-                    nullptr, nullptr, 0, true, &pos, &state, sc);
+                                    std::vector<int64_t> &offsets,
+                                    const std::function<void *(size_t)> &room, FetchScratch *sc) {
+  if (!sc) sc = &g->fs;
+  const int rc = fetch_run(g, st, centers, nq, radius, filter, max_results, true, sc);
+  if (rc) return rc;
+  const long long *off = static_cast<const long long *>(sc->hoff);
+  offsets.assign(off, off + nq + 1);
+  const size_t n = static_cast<size_t>(sc->pending);
+  if (n == 0) return CUBLOX_OK;
+  char *dst = static_cast<char *>(room(13 * n));
+  if (!dst) return fail(CUBLOX_ERR_NOMEM, "fetch: no memory for the samples");
+  CK(cudaMemcpyAsync(dst, sc->fpos, 12 * n, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(dst + 12 * n, sc->fstate, n, cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  return CUBLOX_OK;
 }
 
 size_t cublox_b200::detail::fetch_block_bytes(int centres) {
@@ -1536,6 +1634,9 @@ size_t cublox_b200::detail::fetch_block_bytes(int centres) {
 int cublox_b200::detail::reserve_fetch(FetchScratch *sc, int centres, int64_t samples,
                                        cudaStream_t st) {
   int rc = ensure_fq(sc, st, fetch_block_bytes(centres));
+  if (!rc)
+    rc = ensure_pinned(&sc->hoff, &sc->hoff_bytes,
+                       sizeof(long long) * (static_cast<size_t>(std::max(centres, 0)) + 1));
   if (rc) return rc;
   return ensure_fout(sc, st, samples);
 }
@@ -1544,6 +1645,8 @@ void cublox_b200::detail::free_fetch(FetchScratch *sc) {
   cublox_b200::detail::dfree(sc->fq);
   cublox_b200::detail::dfree(sc->fpos);
   cublox_b200::detail::dfree(sc->fstate);
+  cublox_b200::detail::hfree(sc->hoff);
+  cublox_b200::detail::hfree(sc->hcopy);
   *sc = FetchScratch{};
 }
 
@@ -1560,11 +1663,9 @@ int cublox_grid_fetch_viz(cublox_grid *g, const float center[3], float radius, i
   if (!g || !center || !robot_pos || !n_out || (capacity > 0 && !out_xyzrgb))
     return fail(CUBLOX_ERR_INVALID, "fetch_viz: null argument");
   if (max_points < 0) return fail(CUBLOX_ERR_INVALID, "fetch_viz: negative max_points");
-  int64_t off[2] = {0, 0};
-  int rc = fetch_impl(g, g->stream, center, 1, radius, filter, max_results, nullptr, off,
-                      nullptr, nullptr, std::numeric_limits<int64_t>::max(), true);
+  int rc = fetch_run(g, g->stream, center, 1, radius, filter, max_results, true, &g->fs);
   if (rc) return rc;
-  const int64_t total = off[1];
+  const int64_t total = g->fs.pending;
   if (total == 0 || max_points == 0) return CUBLOX_OK;
   const int64_t cap = std::min<int64_t>(max_points, total);
   if (capacity < cap)
@@ -1617,19 +1718,33 @@ int cublox_grid_fetch(cublox_grid *g, const float center[3], float radius,
                       uint8_t *out_state, int64_t capacity, int64_t *n_out) {
   if (n_out) *n_out = 0;
   if (!g || !center) return fail(CUBLOX_ERR_INVALID, "cublox_grid_fetch: null argument");
-  int64_t kept = 0;
-  int rc = fetch_impl(g, g->stream, center, 1, radius, filter, max_results, &kept, nullptr,
-                      nullptr, nullptr, 0, false);
+  int rc = fetch_run(g, g->stream, center, 1, radius, filter, max_results, true, &g->fs);
   if (rc) return rc;
+  const int64_t kept = g->fs.pending;
   if (kept > capacity)
     return fail(CUBLOX_ERR_INVALID, "cublox_grid_fetch: capacity " + std::to_string(capacity) +
                                         " < " + std::to_string(kept) + " samples");
-  int64_t off[2];
-  rc = fetch_impl(g, g->stream, center, 1, radius, filter, max_results, nullptr, off, out_pos,
-                  out_state, capacity, true);
-  if (rc) return rc;
-  if (n_out) *n_out = off[1];
+  if ((rc = fetch_copy(g, g->stream, &g->fs, out_pos, out_state))) return rc;
+  if (n_out) *n_out = kept;
   return CUBLOX_OK;
+}
+
+int cublox_grid_fetch_begin(cublox_grid *g, const float *centers, int n_centers, float radius,
+                            int filter, int max_results, int64_t *out_offsets) {
+  if (!out_offsets) return fail(CUBLOX_ERR_INVALID, "fetch_begin: null offsets");
+  const int rc = fetch_run(g, g ? g->stream : nullptr, centers, n_centers, radius, filter,
+                           max_results, true, nullptr);
+  if (rc) return rc;
+  const long long *off = static_cast<const long long *>(g->fs.hoff);
+  std::copy(off, off + std::max(n_centers, 0) + 1, out_offsets);
+  return CUBLOX_OK;
+}
+
+int cublox_grid_fetch_read(cublox_grid *g, float *out_pos, uint8_t *out_state, int64_t n) {
+  if (!g) return fail(CUBLOX_ERR_INVALID, "null grid");
+  if (g->fs.pending < 0 || n != g->fs.pending)
+    return fail(CUBLOX_ERR_INVALID, "fetch_read: not the samples of the last fetch_begin");
+  return fetch_copy(g, g->stream, &g->fs, out_pos, out_state);
 }
 
 int cublox_grid_fetch_batch(cublox_grid *g, const float *centers,
@@ -1638,16 +1753,25 @@ int cublox_grid_fetch_batch(cublox_grid *g, const float *centers,
                             float *out_pos, uint8_t *out_state,
                             int64_t capacity) {
   if (!out_offsets) return fail(CUBLOX_ERR_INVALID, "fetch_batch: null offsets");
-  return fetch_impl(g, g ? g->stream : nullptr, centers, n_centers, radius, filter,
-                    max_results, nullptr, out_offsets, out_pos, out_state, capacity, true);
+  const int rc =
+      cublox_grid_fetch_begin(g, centers, n_centers, radius, filter, max_results, out_offsets);
+  if (rc) return rc;
+  if (g->fs.pending > capacity)
+    return fail(CUBLOX_ERR_INVALID, "fetch: output capacity " + std::to_string(capacity) + " < " +
+                                        std::to_string(g->fs.pending) + " samples");
+  return fetch_copy(g, g->stream, &g->fs, out_pos, out_state);
 }
 
 int cublox_grid_fetch_counts(cublox_grid *g, const float *centers,
                              int n_centers, float radius, int filter,
                              int max_results, int64_t *out_counts) {
   if (!out_counts) return fail(CUBLOX_ERR_INVALID, "fetch_counts: null output");
-  return fetch_impl(g, g ? g->stream : nullptr, centers, n_centers, radius, filter,
-                    max_results, out_counts, nullptr, nullptr, nullptr, 0, false);
+  const int rc = fetch_run(g, g ? g->stream : nullptr, centers, n_centers, radius, filter,
+                           max_results, false, nullptr);
+  if (rc) return rc;
+  const long long *off = static_cast<const long long *>(g->fs.hoff);
+  for (int i = 0; i < n_centers; ++i) out_counts[i] = off[i + 1] - off[i];
+  return CUBLOX_OK;
 }
 
 // ---- queries / state access ---------------------------------------------------
@@ -1656,25 +1780,36 @@ int cublox_grid_query_states(cublox_grid *g, const float *xyz, int n,
   if (!g || (n > 0 && (!xyz || !out_state)))
     return fail(CUBLOX_ERR_INVALID, "query_states: null argument");
   if (n <= 0) return CUBLOX_OK;
-  if (n > g->qcap) {
+  // Up to kInPlacePoints the kernel reads the points from, and writes the
+  // states to, pinned host memory: one launch instead of two copies around
+  // it, each with its own start and end (256 points: 26 us -> 12 us).  More
+  // points take the copy engines.
+  constexpr int kInPlacePoints = 1 << 16;
+  const bool in_place = n <= kInPlacePoints;
+  const size_t in_bytes = sizeof(float) * 3 * static_cast<size_t>(n);
+  if (in_place) {
+    const int rc = ensure_pinned(&g->h_query, &g->h_query_bytes, in_bytes + static_cast<size_t>(n));
+    if (rc) return rc;
+    std::memcpy(g->h_query, xyz, in_bytes);
+  } else if (n > g->qcap) {
     CK(cudaStreamSynchronize(g->stream));
     cublox_b200::detail::dfree(g->d_qin);
     cublox_b200::detail::dfree(g->d_qout);
     g->d_qin = nullptr;
     g->d_qout = nullptr;
     g->qcap = 0;
-    if (cublox_b200::detail::dmalloc(&g->d_qin, sizeof(float) * 3 * static_cast<size_t>(n)) != cudaSuccess ||
+    if (cublox_b200::detail::dmalloc(&g->d_qin, in_bytes) != cudaSuccess ||
         cublox_b200::detail::dmalloc(&g->d_qout, static_cast<size_t>(n)) != cudaSuccess) {
       cudaGetLastError();
       return fail(CUBLOX_ERR_NOMEM, "query_states: allocation failed");
     }
     g->qcap = n;
   }
-  CK(cudaMemcpyAsync(g->d_qin, xyz, sizeof(float) * 3 * static_cast<size_t>(n),
-                     cudaMemcpyHostToDevice, g->stream));
+  if (!in_place)
+    CK(cudaMemcpyAsync(g->d_qin, xyz, in_bytes, cudaMemcpyHostToDevice, g->stream));
   QueryParams p{};
   p.occ = g->d_occ;
-  p.xyz = g->d_qin;
+  p.xyz = in_place ? static_cast<const float *>(g->h_query) : g->d_qin;
   p.n = n;
   for (int a = 0; a < 3; ++a) {
     p.win[a] = g->origin_i[a];
@@ -1686,13 +1821,15 @@ int cublox_grid_query_states(cublox_grid *g, const float *xyz, int n,
   p.l_free = g->l_free;
   p.l_occ = g->l_occ;
   p.l_unknown = g->l_unknown;
-  p.out = g->d_qout;
+  p.out = in_place ? static_cast<uint8_t *>(g->h_query) + in_bytes : g->d_qout;
   p.lay = g->lay;
   launch_query(p, g->stream);
   CK_LAUNCH();
-  CK(cudaMemcpyAsync(out_state, g->d_qout, static_cast<size_t>(n), cudaMemcpyDeviceToHost,
-                     g->stream));
+  if (!in_place)
+    CK(cudaMemcpyAsync(out_state, g->d_qout, static_cast<size_t>(n), cudaMemcpyDeviceToHost,
+                       g->stream));
   CK(cudaStreamSynchronize(g->stream));
+  if (in_place) std::memcpy(out_state, p.out, static_cast<size_t>(n));
   return CUBLOX_OK;
 }
 

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -20,6 +21,11 @@ struct FetchScratch {
   float *fpos = nullptr;
   uint8_t *fstate = nullptr;
   int64_t fcap = 0;
+  int64_t pending = -1;  // samples of the last fetch, in fpos and fstate (-1: none)
+  void *hoff = nullptr;  // pinned: the queries' offsets
+  size_t hoff_bytes = 0;
+  void *hcopy = nullptr;  // pinned: samples on their way to pageable memory
+  size_t hcopy_bytes = 0;
 };
 // Bytes of one set of a map's line flags (16-byte loads start on its lines).
 inline size_t flag_bytes(int nlines) { return (static_cast<size_t>(nlines) + 255) & ~size_t(255); }
@@ -109,6 +115,8 @@ struct cublox_grid {
   uint8_t *d_qout = nullptr;
   float *d_qin = nullptr;
   int qcap = 0;
+  void *h_query = nullptr;  // pinned: points and states of a query read in place
+  size_t h_query_bytes = 0;
 };
 
 namespace cublox_b200 {
@@ -185,13 +193,13 @@ int detach_voxels(cublox_grid *g, float *occ_host, VoxelBuffers *out);
 // Give g the buffers *in (same nalloc) and enqueue, on g's stream, the copy
 // of its stored log-odds from occ_host (all unknown if null).
 int attach_voxels(cublox_grid *g, VoxelBuffers *in, const float *occ_host);
-// fetch_batch on stream st (ordered after the grid's work by the caller),
-// outputs sized to the samples found, in the scratch `sc` (the grid's own if
-// null).
+// fetch_batch on stream st (ordered after the grid's work by the caller), in
+// the scratch `sc` (the grid's own if null).  room(bytes) gives the host
+// memory (pinned for a direct copy) for the n samples found: 12 n bytes of
+// positions, then n of states; not called if there are none.
 int fetch_into(cublox_grid *g, cudaStream_t st, const float *centers, int nq, float radius,
                int filter, int max_results, std::vector<int64_t> &offsets,
-               std::vector<float> &pos, std::vector<uint8_t> &state,
-               FetchScratch *sc = nullptr);
+               const std::function<void *(size_t)> &room, FetchScratch *sc = nullptr);
 // Device bytes of the query block of a fetch of that many centres (of up to 2
 // m at 0.1 m; larger boxes grow it).
 size_t fetch_block_bytes(int centres);

@@ -330,29 +330,39 @@ __device__ __forceinline__ int f2i_hostlike(float v) {
                                                     : (-2147483647 - 1);
 }
 
-__global__ void __launch_bounds__(256) query_kernel(const QueryParams p) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.n;
-       i += gridDim.x * blockDim.x) {
-    int g[3];
-    bool in = true;
+// The points and states may sit in pinned host memory: a CTA reads its
+// points as one run of consecutive floats, each once over the bus.
+constexpr int kQueryThreads = 128;
+
+__global__ void __launch_bounds__(kQueryThreads) query_kernel(const QueryParams p) {
+  __shared__ float xyz[3 * kQueryThreads];
+  const int start = blockIdx.x * kQueryThreads, n = min(kQueryThreads, p.n - start);
+  const float *src = p.xyz + 3 * static_cast<size_t>(start);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const float v = p.xyz[3 * static_cast<size_t>(i) + a];
-      const float m = fmul(v, p.inv);
-      g[a] = p.ctr ? f2i_hostlike(fadd(m, v < 0.0f ? -0.5f : 0.5f))
-                   : f2i_hostlike(ffloor(m));
-      in = in && abs(g[a] - p.win[a]) <= p.half[a];
-    }
-    uint8_t st = 0;
-    if (in) {
-      const int h = vox_addr(p.lay, global_to_local(g[0], p.map[0], p.half[0]) + p.half[0],
-                             global_to_local(g[1], p.map[1], p.half[1]) + p.half[1],
-                             global_to_local(g[2], p.map[2], p.half[2]) + p.half[2]);
-      const float l = fadd(p.occ[h], p.l_unknown);
-      st = l >= p.l_occ ? 2 : (l < p.l_free ? 1 : 0);
-    }
-    p.out[i] = st;
+  for (int r = 0; r < 3; ++r) {
+    const int j = r * kQueryThreads + threadIdx.x;
+    if (j < 3 * n) xyz[j] = src[j];
   }
+  __syncthreads();
+  if (static_cast<int>(threadIdx.x) >= n) return;
+  int g[3];
+  bool in = true;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float v = xyz[3 * threadIdx.x + a];
+    const float m = fmul(v, p.inv);
+    g[a] = p.ctr ? f2i_hostlike(fadd(m, v < 0.0f ? -0.5f : 0.5f)) : f2i_hostlike(ffloor(m));
+    in = in && abs(g[a] - p.win[a]) <= p.half[a];
+  }
+  uint8_t st = 0;
+  if (in) {
+    const int h = vox_addr(p.lay, global_to_local(g[0], p.map[0], p.half[0]) + p.half[0],
+                           global_to_local(g[1], p.map[1], p.half[1]) + p.half[1],
+                           global_to_local(g[2], p.map[2], p.half[2]) + p.half[2]);
+    const float l = fadd(p.occ[h], p.l_unknown);
+    st = l >= p.l_occ ? 2 : (l < p.l_free ? 1 : 0);
+  }
+  p.out[start + threadIdx.x] = st;
 }
 
 __global__ void gather_soa_kernel(const float *xyz, int layout, int n,
@@ -625,8 +635,7 @@ void launch_clear(const ClearParams &p, cudaStream_t s) {
 
 void launch_query(const QueryParams &p, cudaStream_t s) {
   if (p.n <= 0) return;
-  int grid = (p.n + 255) / 256;
-  query_kernel<<<grid, 256, 0, s>>>(p);
+  query_kernel<<<(p.n + kQueryThreads - 1) / kQueryThreads, kQueryThreads, 0, s>>>(p);
 }
 
 void launch_gather_soa(const float *xyz, int layout, int n, float *dst,

@@ -29,6 +29,7 @@
 #include <deque>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <unordered_map>
@@ -61,8 +62,8 @@ struct Request {
   int filter = CUBLOX_FILTER_ALL;
   int max_results = 0;
   std::vector<int64_t> offsets;
-  std::vector<float> fpos;
-  std::vector<uint8_t> fstate;
+  int64_t fn = 0;                // samples found
+  std::shared_ptr<char> fresult;  // their positions, then their states
   // progress
   int state = CUBLOX_REQ_QUEUED;
   int error = CUBLOX_OK;
@@ -421,6 +422,20 @@ void defer(cublox_server *s, Request *r) {
   s->maps[r->map]->queue.push_front(r);
 }
 
+// Host memory for a fetch's result: a block of the pinned pool, which the
+// device copies into directly and which goes back when the request is
+// released, or, where the pool has none, pageable memory.
+void *result_room(cublox_server *s, Request *r, size_t bytes) {
+  int cls = -1;
+  if (float *p = s->pinned.take(bytes, &cls))
+    r->fresult = std::shared_ptr<char>(reinterpret_cast<char *>(p), [s, p, cls](char *) {
+      s->pinned.give(p, cls);
+    });
+  else
+    r->fresult = std::shared_ptr<char>(new (std::nothrow) char[bytes], std::default_delete<char[]>());
+  return r->fresult.get();
+}
+
 // Fetches run on their own thread and stream: the job waits (on the device)
 // for the work queued on its map before it, and the map takes no new tick
 // until the fetch is done, so later scans cannot overtake it.
@@ -445,8 +460,10 @@ void fetcher_loop(cublox_server *s) {
     if (!rc)
       rc = cublox_b200::detail::fetch_into(m.g, s->fstream, r->centers.data(),
                                            static_cast<int>(r->centers.size() / 3), r->radius,
-                                           r->filter, r->max_results, r->offsets, r->fpos,
-                                           r->fstate, &s->fscratch);
+                                           r->filter, r->max_results, r->offsets,
+                                           [&](size_t bytes) { return result_room(s, r, bytes); },
+                                           &s->fscratch);
+    r->fn = rc ? 0 : r->offsets.back();
     const std::string msg = rc ? cublox_last_error() : "";
     std::lock_guard<std::mutex> lk(s->mu);
     ++s->stats.fetches;
@@ -913,18 +930,24 @@ int cublox_server_fetch_result(cublox_server *s, int64_t request_id, int64_t *of
                                float *out_pos, uint8_t *out_state, int64_t capacity,
                                int64_t *n_samples) {
   if (!s) return fail(CUBLOX_ERR_INVALID, "null server");
-  std::lock_guard<std::mutex> lk(s->mu);
-  Request *r = find(s, request_id);
-  if (!r || r->kind != kFetch) return fail(CUBLOX_ERR_INVALID, "fetch_result: not a fetch");
-  if (r->state != CUBLOX_REQ_DONE) return fail(CUBLOX_ERR_INVALID, "fetch_result: not done");
-  const int64_t n = static_cast<int64_t>(r->fstate.size());
-  if (n_samples) *n_samples = n;
-  if (offsets) std::copy(r->offsets.begin(), r->offsets.end(), offsets);
-  if (out_pos || out_state) {
+  std::shared_ptr<char> result;  // held while it is copied, outside the lock
+  int64_t n = 0;
+  {
+    std::lock_guard<std::mutex> lk(s->mu);
+    Request *r = find(s, request_id);
+    if (!r || r->kind != kFetch) return fail(CUBLOX_ERR_INVALID, "fetch_result: not a fetch");
+    if (r->state != CUBLOX_REQ_DONE) return fail(CUBLOX_ERR_INVALID, "fetch_result: not done");
+    n = r->fn;
+    if (n_samples) *n_samples = n;
+    if (offsets) std::copy(r->offsets.begin(), r->offsets.end(), offsets);
+    if (!out_pos && !out_state) return CUBLOX_OK;
     if (capacity < n) return fail(CUBLOX_ERR_INVALID, "fetch_result: capacity too small");
-    if (out_pos) std::copy(r->fpos.begin(), r->fpos.end(), out_pos);
-    if (out_state) std::copy(r->fstate.begin(), r->fstate.end(), out_state);
+    result = r->fresult;
   }
+  if (n == 0) return CUBLOX_OK;
+  const size_t bytes = static_cast<size_t>(n);
+  if (out_pos) std::memcpy(out_pos, result.get(), 12 * bytes);
+  if (out_state) std::memcpy(out_state, result.get() + 12 * bytes, bytes);
   return CUBLOX_OK;
 }
 

@@ -226,15 +226,14 @@ class OccupancyGrid : public Grid {
     if (!g_) return out;
     const float c[3] = {center.x(), center.y(), center.z()};
     const int flt = state_filter ? static_cast<int>(*state_filter) : CUBLOX_FILTER_ALL;
-    int64_t n = 0;
-    detail::ok(cublox_grid_fetch_counts(g_, c, 1, radius, flt, max_results, &n),
+    int64_t off[2] = {0, 0};
+    detail::ok(cublox_grid_fetch_begin(g_, c, 1, radius, flt, max_results, off),
                "fetchOccupancyAround");
-    if (n <= 0) return out;
-    std::vector<float> pos(3 * static_cast<size_t>(n));
-    std::vector<uint8_t> st(static_cast<size_t>(n));
-    int64_t got = 0;
-    detail::ok(cublox_grid_fetch(g_, c, radius, flt, max_results, pos.data(), st.data(), n, &got),
-               "fetchOccupancyAround");
+    const int64_t got = off[1];
+    if (got <= 0) return out;
+    std::vector<float> pos(3 * static_cast<size_t>(got));
+    std::vector<uint8_t> st(static_cast<size_t>(got));
+    detail::ok(cublox_grid_fetch_read(g_, pos.data(), st.data(), got), "fetchOccupancyAround");
     out.reserve(static_cast<size_t>(got));
     for (int64_t i = 0; i < got; ++i)
       out.push_back({Eigen::Vector3f(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]),

@@ -214,6 +214,14 @@ int cublox_grid_fetch_batch(cublox_grid *g, const float *centers,
                             int max_results, int64_t *out_offsets,
                             float *out_pos, uint8_t *out_state,
                             int64_t capacity);
+/* The same in two calls, for callers that size their outputs by the number
+ * of samples: begin finds them (out_offsets as above, n_centers + 1 entries)
+ * and keeps them on the device; read copies them out, n = out_offsets[last].
+ * read refuses any other n, and a grid on which another fetch was made since.
+ * No counterpart in the reference.                                          */
+int cublox_grid_fetch_begin(cublox_grid *g, const float *centers, int n_centers, float radius,
+                            int filter, int max_results, int64_t *out_offsets);
+int cublox_grid_fetch_read(cublox_grid *g, float *out_pos, uint8_t *out_state, int64_t n);
 /* Counts only: per-centre sample counts, no samples materialised.         */
 int cublox_grid_fetch_counts(cublox_grid *g, const float *centers,
                              int n_centers, float radius, int filter,

@@ -70,3 +70,47 @@ def test_fetch_makes_room_and_keeps_it():
     assert rc == C.ERR_INVALID and not pos.any()  # too little room: refused, nothing written
     _same(g, o, many[:2], 0.3, -1, 0)
     g.close()
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 65536, 65537])
+def test_query_in_place_and_copied(n):
+    """Point queries where a CTA ends, and on both sides of the number of
+    points that are read in place."""
+    rng = np.random.default_rng(n)
+    g, o, s = _pair((30, 30, 10), False, (7, -3, 2), None, rng)
+    p = (s + rng.uniform(-3.5, 3.5, (n, 3))).astype(np.float32)
+    p[0] = [np.nan, 0, 0]
+    with np.errstate(invalid="ignore"):  # the reference bins on the host: x86 conversion, NaN to INT_MIN
+        q = p * np.float32(1.0 / np.float32(0.1))
+        v = np.where(np.isfinite(q), np.floor(q), -2.0**31).astype(np.int64)
+    half, win = np.array((30, 30, 10)), np.array(o.origin()[0])
+    inside = (np.abs(v - win) <= half).all(1)
+    slot = (v + half) % (2 * half + 1)
+    l = o.occ().reshape(2 * half + 1)[tuple(slot.T)]
+    want = np.where(inside, np.where(l >= np.float32(LO[5]), 2, np.where(l < np.float32(LO[4]), 1, 0)), 0)
+    for _ in range(2):
+        assert np.array_equal(g.query_states(p), want)
+    g.close()
+
+
+def test_fetch_in_two_calls():
+    """begin / read: samples of several copies' sizes, and what read refuses."""
+    import ctypes
+
+    rng = np.random.default_rng(2)
+    g, o, s = _pair((60, 60, 20), False, (0, 0, 0), None, rng)
+    L = C.lib()
+    i64, f = ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_float)
+    c = np.ascontiguousarray(s + rng.uniform(-1, 1, (40, 3)), np.float32)
+    off = np.zeros(41, np.int64)
+    for n, r in ((1, 0.3), (40, 0.5), (40, 2.0)):  # one piece, one copy, several threads
+        assert L.cublox_grid_fetch_begin(g._h, c.ctypes.data_as(f), n, r, -1, 0, off.ctypes.data_as(i64)) == C.OK
+        pos = np.empty((off[n], 3), np.float32)
+        assert L.cublox_grid_fetch_read(g._h, pos.ctypes.data_as(f), None, int(off[n]) + 1) == C.ERR_INVALID
+        for _ in range(2):
+            assert L.cublox_grid_fetch_read(g._h, pos.ctypes.data_as(f), None, int(off[n])) == C.OK
+        want = np.concatenate([o.fetch(x, r, -1, 0)[0] for x in c[:n]])
+        assert np.array_equal(pos.view(np.uint32), want.view(np.uint32))
+        g.fetch_counts(c, r)
+        assert L.cublox_grid_fetch_read(g._h, pos.ctypes.data_as(f), None, int(off[n])) == C.ERR_INVALID
+    g.close()
