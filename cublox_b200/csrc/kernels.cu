@@ -187,6 +187,15 @@ __global__ void __launch_bounds__(kListThreads, 4) fold_list_kernel(const ApplyP
   const uint4 fh = load_line_flags(p.hot, start, count);
   const int2 n = build_line_list(line_flag_bits(f), line_flag_bits(fh), L, p.dirty, p.hot, start, count);
   uint32_t touched = fold_line_list<3, false>(v, L, n, start);
+  // voxels past the last whole line (arrays without padding)
+  if (blockIdx.x == gridDim.x - 1) {
+    const int h = (p.nlines << kLineShift) + static_cast<int>(threadIdx.x);
+    if (h < p.vnum && p.cnt[h]) {
+      fold(p, h, p.cnt[h]);
+      p.cnt[h] = 0u;
+      ++touched;
+    }
+  }
   if (kStats) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
@@ -560,15 +569,15 @@ void launch_step_count(const RayParams &p, cudaStream_t s) {
 
 void launch_apply(const ApplyParams &p, cudaStream_t s) {
   if (p.variant == 2) {
-    if (p.nlines <= 0) return;
+    if (p.nlines <= 0 && p.vnum <= 0) return;
     // items of up to kPlainItemLines lines, smaller for small maps so that
     // every SM gets some (a multiple of 16 lines keeps the 16-byte flag
     // loads aligned)
     const int cap = sm_count() * 4;
     int item_lines = (p.nlines + cap - 1) / cap;
-    item_lines = ((item_lines + 255) / 256) * 256;
+    item_lines = item_lines > 0 ? ((item_lines + 255) / 256) * 256 : 256;
     if (item_lines > kPlainItemLines) item_lines = kPlainItemLines;
-    const int grid = (p.nlines + item_lines - 1) / item_lines;
+    const int grid = p.nlines > 0 ? (p.nlines + item_lines - 1) / item_lines : 1;
     if (p.stats)
       fold_list_kernel<true><<<grid, kListThreads, 0, s>>>(p, item_lines);
     else

@@ -6,21 +6,27 @@
 // budget), or code that runs inside a host framework which hands it only a
 // stream and buffers it owns (an inference-engine plugin's enqueue step, a
 // pooled multi-tenant server).  Such a caller owns the map buffers and the
-// points; this entry point owns nothing but a fixed scratch area for
-// sorting the rays by direction, which lives in a file-scope __device__
-// array (every GPU that loads the library holds it until the process exits).
+// points; this entry point owns nothing but a fixed scratch area, which
+// lives in a file-scope __device__ array (every GPU that loads the library
+// holds it until the process exits).
+//
+// Maps of up to 134M voxels are walked in direction order (cone_walk.cuh) and
+// folded by flagged lines (fold.cuh), with the line flags in the scratch.
+// Larger ones, those too wide for that walk's step table, and hit counters
+// that are not 16-byte aligned take the direction-binned walk, with its sorted
+// rays in the scratch, and a sweep of every counter (a 65,536-ray scan into
+// 701 x 701 x 151 voxels: 505 us; in direction order 267).
 //
 // The scratch is shared by every call on a device and keeps whatever the
-// last call left in it.  The direction histogram is cleared at the start of
-// each call; every other scratch word is fully overwritten before it is
-// read.  Calls whose GPU work overlaps (different streams, or different host
+// last call left in it.  The line flags or the direction histogram are
+// cleared at the start of each call; every other scratch word is fully
+// overwritten before it is read.  Calls whose GPU work overlaps (different streams, or different host
 // threads, at the same time) race on the scratch and must not be issued.
 //
-// The direction-binned walk and the counter sweep used here have no
-// device-side check that can fail (every index they form is in range by
-// construction), so this entry point reports no device error word: the
-// kernels are given none (RayParams::err is null, and neither kernel
-// dereferences it).
+// The walks and folds used here have no device-side check that can fail
+// (every index they form is in range by construction), so this entry point
+// reports no device error word: the kernels are given none (RayParams::err is
+// null, and none of them dereferences it).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -29,6 +35,7 @@
 #include <string>
 
 #include "../../include/cublox_b200.h"
+#include "cone_walk.cuh"
 #include "exact_fp.cuh"
 #include "kernels.cuh"
 
@@ -44,7 +51,10 @@ constexpr size_t kOffHist = sizeof(int) * kMaxPoints;
 constexpr size_t kOffCursor = kOffHist + sizeof(int) * kBinsWords;
 constexpr size_t kOffSorted = kOffCursor + sizeof(int) * kBinsWords;
 static_assert(kOffSorted % 16 == 0, "sorted points must start on a 16-byte boundary");
-constexpr size_t kScratchBytes = kOffSorted + sizeof(float) * 3 * kMaxPoints;
+constexpr size_t kSortBytes = kOffSorted + sizeof(float) * 3 * kMaxPoints;
+// Or: flags of up to kFlagLines lines | flags of lines with a hit
+constexpr size_t kFlagLines = size_t(1) << 22;
+constexpr size_t kScratchBytes = 2 * kFlagLines > kSortBytes ? 2 * kFlagLines : kSortBytes;
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -57,6 +67,32 @@ thread_local std::string g_noalloc_err;
 int noalloc_fail(int code, const std::string &msg) {
   g_noalloc_err = msg;
   return code;
+}
+
+// The fold of the scan that `p` walked: variant 2 by flagged lines, 1 a sweep.
+int fold(const cublox_map_view *map, const RayParams &p, int variant, int lines, cudaStream_t s) {
+  ApplyParams a{};
+  a.occ = map->occ;
+  a.cnt = map->cnt;
+  a.hit = map->hit;
+  a.vnum = p.vnum;
+  a.l_hit = map->l_hit;
+  a.l_miss = map->l_miss;
+  a.l_min = map->l_min;
+  a.l_max = map->l_max;
+  a.l_unknown = 0.0f;
+  a.fp = kFpPinned;
+  a.stats = nullptr;
+  a.variant = variant;
+  a.dirty = p.dirty;
+  a.hot = p.hot;
+  a.nlines = lines;
+  launch_apply(a, s);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess)
+    return noalloc_fail(CUBLOX_ERR_CUDA, std::string("cublox_integrate_noalloc: fold: ") +
+                                             cudaGetErrorString(e));
+  return CUBLOX_OK;
 }
 
 }  // namespace
@@ -142,12 +178,30 @@ int cublox_integrate_noalloc(const cublox_map_view *map, const float *xyz_soa, i
   p.hit = map->hit;
   p.stats = nullptr;
   p.err = nullptr;  // no check on this path can fail (file comment)
-  // the caller's arrays are in the reference's hash order, and have no line
-  // flags: the fold below sweeps every counter
+  // the caller's arrays are in the reference's hash order, and bring no line
+  // flags
   p.lay.bs[0] = mapsz[1] * mapsz[2];
   p.lay.bs[1] = mapsz[2];
   p.lay.bs[2] = 1;
   p.dirty = p.hot = nullptr;
+
+  // lines of 32 voxels in full, and the last, partial one
+  const int64_t lines = vnum >> kLineShift;
+  const size_t flags = (static_cast<size_t>(lines) + 1 + 255) & ~size_t(255);
+  const auto aligned = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+  if (flags <= kFlagLines && cone_takes(mapsz, vnum) && aligned(map->occ) && aligned(map->cnt) &&
+      aligned(map->hit)) {
+    p.dirty = base;
+    p.hot = base + flags;
+    if ((e = cudaMemsetAsync(base, 0, 2 * flags, s)) == cudaSuccess) {
+      launch_raycast_cone(p, s);
+      e = cudaGetLastError();
+    }
+    if (e != cudaSuccess)
+      return noalloc_fail(CUBLOX_ERR_CUDA, std::string("cublox_integrate_noalloc: raycast: ") +
+                                               cudaGetErrorString(e));
+    return fold(map, p, 2, static_cast<int>(lines), s);
+  }
 
   BinnedScratch b{reinterpret_cast<int *>(base), reinterpret_cast<int *>(base + kOffHist),
                   reinterpret_cast<int *>(base + kOffCursor),
@@ -158,25 +212,7 @@ int cublox_integrate_noalloc(const cublox_map_view *map, const float *xyz_soa, i
   if (e != cudaSuccess)
     return noalloc_fail(CUBLOX_ERR_CUDA, std::string("cublox_integrate_noalloc: raycast: ") +
                                              cudaGetErrorString(e));
-  ApplyParams a{};
-  a.occ = map->occ;
-  a.cnt = map->cnt;
-  a.hit = map->hit;
-  a.vnum = p.vnum;
-  a.l_hit = map->l_hit;
-  a.l_miss = map->l_miss;
-  a.l_min = map->l_min;
-  a.l_max = map->l_max;
-  a.l_unknown = 0.0f;
-  a.fp = kFpPinned;
-  a.stats = nullptr;
-  a.variant = 1;
-  launch_apply(a, s);
-  e = cudaGetLastError();
-  if (e != cudaSuccess)
-    return noalloc_fail(CUBLOX_ERR_CUDA, std::string("cublox_integrate_noalloc: fold: ") +
-                                             cudaGetErrorString(e));
-  return CUBLOX_OK;
+  return fold(map, p, 1, 0, s);
 }
 
 }  // extern "C"

@@ -488,7 +488,7 @@ int cublox_server_scratch_bytes(const cublox_server_config *cfg, uint64_t *bytes
  * first-run origin snap: origin_index is used as given), enqueues on
  * `stream` (a cudaStream_t, NULL for the default stream) and returns.
  *
- * Its only scratch is a fixed area of about 4 MiB in a file-scope device
+ * Its only scratch is a fixed area of 8 MiB in a file-scope device
  * array that every GPU loading this library holds until exit; it allocates
  * nothing and calls no allocating routine.  At most
  * CUBLOX_NOALLOC_MAX_POINTS points per call; more are rejected with
