@@ -378,19 +378,24 @@ __global__ void __launch_bounds__(512, 2) batch_walk_flat_kernel(const MapDesc *
   }
 }
 
-// One cone walk item (cone_walk.cuh): at most kRays = blockDim.x rays, one a
-// thread, ordered by direction.  `map` is the map whose table is in `table`
-// (-1: none).  Ends with a CTA barrier.
-template <int kRays>
+// One cone walk item (cone_walk.cuh): at most kRays = kKeys blockDim.x rays,
+// ordered by direction.  `map` is the map whose table is in `table` (-1:
+// none).  Ends with a CTA barrier.
+template <int kRays, int kKeys>
 __device__ __forceinline__ void walk_item_cone(const MapDesc *maps, const WalkItem &item, int *table,
                                                int &map, ConeItem<kRays> &ci) {
   const RayParams &p = maps[item.map].ray;
   if (item.map != map) cone_table(p, table);  // cone_order's barriers follow
   map = item.map;
-  const int r = cone_order<kRays>(p, item.start, item.count, ci);
+  int ray[kKeys];
+  cone_order<kRays, kKeys>(p, item.start, item.count, ci, ray);
   uint32_t rays = 0, incs = 0, hits = 0;
-  cone_walk(p, table, r >= 0, r >= 0 ? ci.x[r] : 0.0f, r >= 0 ? ci.y[r] : 0.0f,
-            r >= 0 ? ci.z[r] : 0.0f, rays, incs, hits);
+#pragma unroll 1
+  for (int k = 0; k < kKeys; ++k) {
+    const int r = k ? ray[kKeys - 1] : ray[0];
+    cone_walk(p, table, r >= 0, r >= 0 ? ci.x[r] : 0.0f, r >= 0 ? ci.y[r] : 0.0f,
+              r >= 0 ? ci.z[r] : 0.0f, rays, incs, hits);
+  }
   if (p.stats) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -408,10 +413,9 @@ __device__ __forceinline__ void walk_item_cone(const MapDesc *maps, const WalkIt
 }
 
 // Persistent cone walk: CTAs take items of kRays rays from counters[0].
-template <int kRays>
-__global__ void __launch_bounds__(kRays, 1024 / kRays) batch_walk_cone_kernel(const MapDesc *maps,
-                                                                            const WalkItem *items,
-                                                                            int *counters) {
+template <int kRays, int kKeys, int kMinCtas>
+__global__ void __launch_bounds__(kRays / kKeys, kMinCtas)
+    batch_walk_cone_kernel(const MapDesc *maps, const WalkItem *items, int *counters) {
   extern __shared__ uint32_t smem[];
   __shared__ ConeItem<kRays> ci;
   __shared__ int s_item;
@@ -423,7 +427,7 @@ __global__ void __launch_bounds__(kRays, 1024 / kRays) batch_walk_cone_kernel(co
     __syncthreads();
     const int it = s_item;
     if (it >= n_items) break;
-    walk_item_cone<kRays>(maps, items[it], table, map, ci);
+    walk_item_cone<kRays, kKeys>(maps, items[it], table, map, ci);
   }
 }
 
@@ -588,12 +592,12 @@ struct Shape {
   int min_ctas;  // 2: registers capped for two CTAs per SM (cube <= 16)
   int refill;    // 1: two-phase items, lanes refilled from a far-state queue
   int flat;      // 1: S x S x S/2 cube, two 512-thread CTAs per SM
-  int cone;      // 1: cone walk, one ray a thread in direction order (cone_walk.cuh)
+  int cone;      // 1: cone walk, rays in direction order, one or two a thread (cone_walk.cuh)
 };
 
 const Shape kShapes[] = {{0, 512, 512, 0, 1, 0, 0, 1},          {32, 1024, 1024, 0, 1, 0, 0, 0},
                          {0, 256, 256, 0, 1, 0, 0, 1},          {0, 1024, 1024, 0, 1, 0, 0, 1},
-                         {32, 512, 512, 0, 1, 0, 0, 0},         {16, 1024, 1024, 0, 2, 0, 0, 0},
+                         {0, 512, 256, 0, 1, 0, 0, 1},          {16, 1024, 1024, 0, 2, 0, 0, 0},
                          {32, 1024, 1024, 1, 1, 0, 0, 0},       {16, 512, 512, 1, 1, 0, 0, 0},
                          {32, kRefillRays, 512, 0, 1, 1, 0, 0}, {16, kRefillRays, 512, 0, 1, 1, 0, 0},
                          {32, 512, 512, 0, 2, 0, 1, 0},         {32, 256, 512, 0, 2, 0, 1, 0},
@@ -602,18 +606,20 @@ const Shape kShapes[] = {{0, 512, 512, 0, 1, 0, 0, 1},          {32, 1024, 1024,
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 constexpr int kWideShape = 10;  // walks the maps that the cone walk does not take (cone_takes)
 
-// The tuner's candidates: the cone walk's item sizes with the default voxel
-// layout (8 x 4 x 1 bricks), its usual size with 4 x 8 x 1 and 4 x 4 x 2
-// bricks, and the fastest of the shapes with a counter cube.  The cone walk
-// has been the fastest on every workload measured (8 README-scale maps: 0.64
-// ms against 1.16 ms for shape 10; 32 maps of three sizes: 1.16 against 3.19),
-// so the other shapes and the reference's hash order are no longer timed;
-// all stay selectable.  A candidate with another layout moves every grid of
-// the update to it first.
+// The tuner's candidates: the cone walk's item forms with the default voxel
+// layout (8 x 4 x 1 bricks), its usual one with 4 x 8 x 1 and 4 x 4 x 2
+// bricks, and the fastest of the shapes with a counter cube.  Two rays a
+// thread (shape 4: smaller CTAs, each warp a long row of rays and a short one)
+// suit batches of many items (32 maps of three sizes: walk 1.09 ms, shape 0
+// 1.20, shape 10 3.19), one ray a thread those of few (8 README-scale maps:
+// 0.73, 0.64, 1.16).  The other shapes and the reference's hash order have
+// not been the fastest on any workload measured and are not timed; all stay
+// selectable.  A candidate with another layout moves every grid of the update
+// to it first.
 struct Candidate {
   int shape, layout;
 };
-const Candidate kCandidates[] = {{0, 320}, {2, 320}, {3, 320}, {0, 230}, {0, 221}, {10, 320}};
+const Candidate kCandidates[] = {{0, 320}, {2, 320}, {4, 320}, {0, 230}, {0, 221}, {10, 320}};
 constexpr int kNumCandidates = sizeof(kCandidates) / sizeof(kCandidates[0]);
 
 int sm_count_batch() {
@@ -642,9 +648,11 @@ const void *shape_kernel_s(const Shape &sh) {
 // The walk (or fused) kernel of a shape.
 const void *shape_kernel(const Shape &sh) {
   if (sh.cone)
-    return sh.block == 1024  ? reinterpret_cast<const void *>(batch_walk_cone_kernel<1024>)
-           : sh.block == 512 ? reinterpret_cast<const void *>(batch_walk_cone_kernel<512>)
-                             : reinterpret_cast<const void *>(batch_walk_cone_kernel<256>);
+    return sh.rays == 1024  ? reinterpret_cast<const void *>(batch_walk_cone_kernel<1024, 1, 1>)
+           : sh.rays == 256 ? reinterpret_cast<const void *>(batch_walk_cone_kernel<256, 1, 4>)
+           : sh.block == 512
+               ? reinterpret_cast<const void *>(batch_walk_cone_kernel<512, 1, 2>)
+               : reinterpret_cast<const void *>(batch_walk_cone_kernel<512, 2, 5>);
   return sh.cube >= 32 ? shape_kernel_s<32>(sh)
                        : (sh.cube >= 16 ? shape_kernel_s<16>(sh) : shape_kernel_s<0>(sh));
 }

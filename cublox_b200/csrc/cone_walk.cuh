@@ -106,43 +106,67 @@ __device__ __forceinline__ uint32_t cone_place(float dx, float dy, float dz) {
 }
 
 // Reads the item's points (each once: they may sit in host memory) and
-// sorts its rays by direction: a bitonic sort of one key per thread,
-// exchanges within a warp by shuffle.  blockDim.x == kRays, a power of two
-// of at least 32.  Returns this thread's ray (its place in the item), -1
-// past the item's rays.  Contains CTA barriers.
-template <int kRays>
-__device__ __forceinline__ int cone_order(const RayParams &p, int start, int count,
-                                          ConeItem<kRays> &it) {
-  static_assert((kRays & (kRays - 1)) == 0 && kRays >= 32 && kRays <= 1024, "a CTA's worth");
+// sorts its rays by direction: a bitonic sort of kKeys keys per thread (the
+// places t and t + kRays / 2 of the item for two), exchanges within a warp by
+// shuffle.  blockDim.x == kRays / kKeys, a power of two of at least 32.
+// ray[r] is then the ray (its place in the item) that came to this thread's
+// r-th place, -1 past the item's rays: a warp's threads hold 32 neighbours,
+// and with two keys another 32 from half the item's rows away.  An item
+// without a finite point (most of a depth image's sky) is not sorted: all its
+// threads get -1.  Contains CTA barriers.
+template <int kRays, int kKeys>
+__device__ __forceinline__ void cone_order(const RayParams &p, int start, int count,
+                                           ConeItem<kRays> &it, int (&ray)[kKeys]) {
+  constexpr int kThreads = kRays / kKeys;
+  static_assert((kRays & (kRays - 1)) == 0 && kThreads >= 32 && kRays <= 1024 && kKeys <= 2,
+                "a CTA's worth");
   const int t = threadIdx.x;
-  uint32_t key = 0xffffffffu;
-  if (t < count) {
-    const size_t k = static_cast<size_t>(start + t) * p.stride;
-    const float x = p.x[k], y = p.y[k], z = p.z[k];
-    it.x[t] = x;
-    it.y[t] = y;
-    it.z[t] = z;
-    key = (cone_place(x - p.o[0], y - p.o[1], z - p.o[2]) << 10) | t;
+  uint32_t key[kKeys];
+  bool finite = false;
+#pragma unroll
+  for (int r = 0; r < kKeys; ++r) {
+    const int e = t + r * kThreads;
+    key[r] = 0xffffffffu;
+    ray[r] = -1;
+    if (e < count) {
+      const size_t k = static_cast<size_t>(start + e) * p.stride;
+      const float x = p.x[k], y = p.y[k], z = p.z[k];
+      it.x[e] = x;
+      it.y[e] = y;
+      it.z[e] = z;
+      key[r] = (cone_place(x - p.o[0], y - p.o[1], z - p.o[2]) << 10) | e;
+      finite = finite || isfinite(x + y + z);  // a sum out of range: no finite length
+    }
   }
+  if (!__syncthreads_or(finite)) return;
 #pragma unroll
   for (int len = 2; len <= kRays; len <<= 1) {
 #pragma unroll
     for (int d = len >> 1; d > 0; d >>= 1) {
-      uint32_t other;
-      if (d >= 32) {
+      if (d >= 32 && d < kThreads) {
         __syncthreads();
-        it.key[t] = key;
+#pragma unroll
+        for (int r = 0; r < kKeys; ++r) it.key[t + r * kThreads] = key[r];
         __syncthreads();
-        other = it.key[t ^ d];
-      } else {
-        other = __shfl_xor_sync(0xffffffffu, key, d);
       }
-      const bool up = (t & len) == 0, low = (t & d) == 0;
-      key = (up == low) ? min(key, other) : max(key, other);
+      uint32_t other[kKeys];
+#pragma unroll
+      for (int r = 0; r < kKeys; ++r)
+        other[r] = d == kThreads ? key[kKeys - 1 - r]
+                   : d >= 32     ? it.key[(t + r * kThreads) ^ d]
+                                 : __shfl_xor_sync(0xffffffffu, key[r], d);
+#pragma unroll
+      for (int r = 0; r < kKeys; ++r) {
+        const int e = t + r * kThreads;
+        const bool up = (e & len) == 0, low = (e & d) == 0;
+        key[r] = (up == low) ? min(key[r], other[r]) : max(key[r], other[r]);
+      }
     }
   }
   __syncthreads();
-  return key == 0xffffffffu ? -1 : static_cast<int>(key & 0x3ffu);
+#pragma unroll
+  for (int r = 0; r < kKeys; ++r)
+    ray[r] = key[r] == 0xffffffffu ? -1 : static_cast<int>(key[r] & 0x3ffu);
 }
 
 // ---- the walk ----

@@ -18,7 +18,9 @@ __global__ void __launch_bounds__(kRays, 1024 / kRays)
   __shared__ ConeItem<kRays> ci;
   cone_table(p, table);  // cone_order's barriers follow
   const int start = blockIdx.x * kRays;
-  const int r = cone_order<kRays>(p, start, min(kRays, p.n - start), ci);
+  int ray[1];
+  cone_order<kRays, 1>(p, start, min(kRays, p.n - start), ci, ray);
+  const int r = ray[0];
   uint32_t rays = 0, incs = 0, hits = 0;
   cone_walk(p, table, r >= 0, r >= 0 ? ci.x[r] : 0.0f, r >= 0 ? ci.y[r] : 0.0f,
             r >= 0 ? ci.z[r] : 0.0f, rays, incs, hits);
@@ -47,11 +49,11 @@ void launch(const RayParams &p, cudaStream_t s) {
 
 // Rays per item: as many as leave 256 items, so that every SM has some (the
 // longest ray of an item sets its time), 64 to 512.  Wider items put more
-// neighbours into a warp's rows.  Walk times in us at 64 / 128 / 256 / 512
-// rays (the split walk with its plan: last): 16-beam scan of 16,384 rays 32 /
-// 37 / 39 / 46 (78); 64 beams, 65,536 rays 186 / 148 / 119 / 116 (216); 128
-// beams, 262,144 rays 587 / 570 / 455 / 398 (933); 640 x 480 depth image 68 /
-// 61 / 63 / 68 (205).
+// neighbours into a warp's rows.  Walk times in us at 64 / 128 / 256 / 512 /
+// 1,024 rays (the split walk with its plan: last): 16-beam scan of 16,384 rays
+// 32 / 37 / 39 / 46 / - (78); 64 beams, 65,536 rays 186 / 148 / 119 / 116 /
+// 179 (216); 128 beams, 262,144 rays 587 / 570 / 455 / 398 / 377 (933); 640 x
+// 480 depth image, 307,200 rays 68 / 61 / 63 / 68 / 74 (205).
 void launch_raycast_cone(const RayParams &p, cudaStream_t s) {
   if (p.n <= 0) return;
   const int fit = p.n / 256;

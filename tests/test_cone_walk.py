@@ -13,7 +13,7 @@ import oracle as O
 pytestmark = pytest.mark.gpu
 
 LO = C.yaml_log_odds()
-SHAPES = (0, 2, 3)  # batch launch shapes that walk in direction order
+SHAPES = (0, 2, 3, 4)  # batch launch shapes that walk in direction order
 
 
 def _rays(rng, n, sensor, reach):
@@ -32,6 +32,8 @@ def _clouds(rng, n, sensor):
     p[: min(n, len(special))] = np.asarray(special, np.float32)[: min(n, len(special))]
     if n > 600:
         p[-200:] = p[-1]  # many equal rays
+    if n > 2000:
+        p[600:1800] = np.nan  # items without a point
     return p
 
 
@@ -94,7 +96,7 @@ def test_map_too_wide_for_the_step_table():
     b.close()
 
 
-@pytest.mark.parametrize("n", [1, 63, 64, 65, 4096, 32767, 32769, 65537, 131073])
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 4096, 32767, 32769, 65537, 131073, 262144])
 @pytest.mark.parametrize("source", ["host", "device", "device_soa"])
 def test_single_grid_items(n, source):
     """One grid's update at the sizes where its items get wider."""
