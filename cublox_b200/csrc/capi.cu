@@ -1573,6 +1573,7 @@ static int copy_out(cublox_grid *g, cudaStream_t st, FetchScratch *sc,
     if (e != cudaSuccess) error = e;
   };
   std::vector<std::thread> helpers;
+  helpers.reserve(static_cast<size_t>(threads));
   int prev = -1;
   if (cudaGetDevice(&prev) != cudaSuccess) cudaGetLastError();
   try {
@@ -1626,9 +1627,10 @@ int cublox_b200::detail::fetch_into(cublox_grid *g, cudaStream_t st, const float
 }
 
 size_t cublox_b200::detail::fetch_block_bytes(int centres) {
-  // boxes of 48 x 48 columns (2 m at 0.1 m), overlapping 7 tiles along x
+  // boxes of 32 x 32 columns of up to 32 levels (1.5 m at 0.1 m), overlapping
+  // 5 tiles along x
   const size_t n = static_cast<size_t>(std::max(centres, 0));
-  return FetchBlock(n, 7 * n, 48 * 48 * n, 2 * 48 * 48 * n, 48 * n).bytes;
+  return FetchBlock(n, 5 * n, 32 * 32 * n, 32 * 32 * n, 32 * n).bytes;
 }
 
 int cublox_b200::detail::reserve_fetch(FetchScratch *sc, int centres, int64_t samples,
@@ -1785,7 +1787,7 @@ int cublox_grid_query_states(cublox_grid *g, const float *xyz, int n,
   // it, each with its own start and end (256 points: 26 us -> 12 us).  More
   // points take the copy engines.
   constexpr int kInPlacePoints = 1 << 16;
-  const bool in_place = n <= kInPlacePoints;
+  const bool in_place = n <= kInPlacePoints && mem_kind(xyz) != 2 && mem_kind(out_state) != 2;
   const size_t in_bytes = sizeof(float) * 3 * static_cast<size_t>(n);
   if (in_place) {
     const int rc = ensure_pinned(&g->h_query, &g->h_query_bytes, in_bytes + static_cast<size_t>(n));

@@ -200,8 +200,8 @@ int attach_voxels(cublox_grid *g, VoxelBuffers *in, const float *occ_host);
 int fetch_into(cublox_grid *g, cudaStream_t st, const float *centers, int nq, float radius,
                int filter, int max_results, std::vector<int64_t> &offsets,
                const std::function<void *(size_t)> &room, FetchScratch *sc = nullptr);
-// Device bytes of the query block of a fetch of that many centres (of up to 2
-// m at 0.1 m; larger boxes grow it).
+// Device bytes of the query block of a fetch of that many centres (of up to
+// 1.5 m at 0.1 m; larger boxes grow it).
 size_t fetch_block_bytes(int centres);
 // Size `sc` for fetches of up to `centres` centres and `samples` samples, so
 // that such fetches allocate nothing.
