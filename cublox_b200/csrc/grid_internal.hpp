@@ -51,7 +51,7 @@ struct cublox_grid {
   int recenter_mode = 0;
   bool stats_on = false;
   // kernel options (cublox_grid_set_option)
-  int opt_raycast = 2;  // 0 thread per ray, 1 binned warp walk, 2 split walk
+  int opt_raycast = 2;  // 0 thread per ray, 1 binned warp walk, 2 direction order or split walk
   int opt_seg = 64;     // split walk: target in-window steps per lane
   int opt_fold = 2;     // 0 scalar sweep, 1 vector sweep, flagged lines: 2 lists, 3 per warp
   int opt_block = 512;  // split walk CTA size

@@ -126,7 +126,7 @@ int cublox_grid_get_fp_mode(const cublox_grid *g, unsigned *mode);
 #define CUBLOX_OPT_FOLD 6    /* fold: 0 scalar sweep of every counter, 1
                                 16-byte sweep; only the 32-voxel lines the
                                 scan flagged: 2 (default) compacted into a
-                                list per 4096 lines, 3 read 32 flags at a
+                                list per 1024 lines, 3 read 32 flags at a
                                 time per warp                              */
 #define CUBLOX_OPT_BLOCK 7   /* split walk CTA size: 256, 512, 1024         */
 #define CUBLOX_OPT_CONTIGUOUS 8 /* split walk: each CTA walks one run of
