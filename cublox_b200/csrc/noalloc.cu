@@ -12,16 +12,18 @@
 //
 // Maps of up to 134M voxels are walked in direction order (cone_walk.cuh) and
 // folded by flagged lines (fold.cuh), with the line flags in the scratch.
-// Larger ones, those too wide for that walk's step table, and hit counters
-// that are not 16-byte aligned take the direction-binned walk, with its sorted
-// rays in the scratch, and a sweep of every counter (a 65,536-ray scan into
-// 701 x 701 x 151 voxels: 505 us; in direction order 267).
+// Larger ones, those too wide for that walk's step table, and arrays that are
+// not 16-byte aligned take the direction-binned walk, with its sorted rays in
+// the scratch, and a sweep of every counter (a 65,536-ray scan into
+// 701 x 701 x 151 voxels: 505 us; in direction order 267), whose accesses are
+// as wide as the arrays' alignment allows (fold_sweep).
 //
 // The scratch is shared by every call on a device and keeps whatever the
 // last call left in it.  The line flags or the direction histogram are
 // cleared at the start of each call; every other scratch word is fully
-// overwritten before it is read.  Calls whose GPU work overlaps (different streams, or different host
-// threads, at the same time) race on the scratch and must not be issued.
+// overwritten before it is read.  Calls whose GPU work overlaps (different
+// streams, or different host threads, at the same time) race on the scratch
+// and must not be issued.
 //
 // The walks and folds used here have no device-side check that can fail
 // (every index they form is in range by construction), so this entry point
@@ -69,13 +71,20 @@ int noalloc_fail(int code, const std::string &msg) {
   return code;
 }
 
-// The fold of the scan that `p` walked: variant 2 by flagged lines, 1 a sweep.
-int fold(const cublox_map_view *map, const RayParams &p, int variant, int lines, cudaStream_t s) {
+bool aligned(const void *q, uintptr_t bytes) {
+  return (reinterpret_cast<uintptr_t>(q) & (bytes - 1)) == 0;
+}
+
+// The fold of voxels [first, first + n) of the scan that `p` walked: variant 2
+// by flagged lines, 1 a sweep that reads counters and stored values 16 bytes
+// at a time, 0 one that reads only the counters so.
+int fold(const cublox_map_view *map, const RayParams &p, int first, int n, int variant, int lines,
+         cudaStream_t s) {
   ApplyParams a{};
-  a.occ = map->occ;
-  a.cnt = map->cnt;
-  a.hit = map->hit;
-  a.vnum = p.vnum;
+  a.occ = map->occ + first;
+  a.cnt = map->cnt + first;
+  a.hit = map->hit + first;
+  a.vnum = n;
   a.l_hit = map->l_hit;
   a.l_miss = map->l_miss;
   a.l_min = map->l_min;
@@ -93,6 +102,18 @@ int fold(const cublox_map_view *map, const RayParams &p, int variant, int lines,
     return noalloc_fail(CUBLOX_ERR_CUDA, std::string("cublox_integrate_noalloc: fold: ") +
                                              cudaGetErrorString(e));
   return CUBLOX_OK;
+}
+
+// A sweep of all voxels.  Stored values that are not 16-byte aligned are
+// accessed one by one; of counters that are not, the few before the first
+// aligned one are folded by a launch of their own, which has no whole group of
+// four.
+int fold_sweep(const cublox_map_view *map, const RayParams &p, cudaStream_t s) {
+  if (aligned(map->occ, 16) && aligned(map->cnt, 16)) return fold(map, p, 0, p.vnum, 1, 0, s);
+  int lead = static_cast<int>((0 - reinterpret_cast<uintptr_t>(map->cnt)) & 15) / 4;
+  if (lead > p.vnum) lead = p.vnum;
+  const int rc = lead ? fold(map, p, 0, lead, 0, 0, s) : CUBLOX_OK;
+  return rc || lead == p.vnum ? rc : fold(map, p, lead, p.vnum - lead, 0, 0, s);
 }
 
 }  // namespace
@@ -129,6 +150,9 @@ int cublox_integrate_noalloc(const cublox_map_view *map, const float *xyz_soa, i
     vnum *= ms;
   }
   if (n == 0) return CUBLOX_OK;
+  if (!aligned(map->occ, 4) || !aligned(map->cnt, 4) || !aligned(map->hit, 4) || !aligned(xyz_soa, 4))
+    return noalloc_fail(CUBLOX_ERR_INVALID,
+                        "cublox_integrate_noalloc: an array does not start on a 4-byte boundary");
 
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -188,9 +212,8 @@ int cublox_integrate_noalloc(const cublox_map_view *map, const float *xyz_soa, i
   // lines of 32 voxels in full, and the last, partial one
   const int64_t lines = vnum >> kLineShift;
   const size_t flags = (static_cast<size_t>(lines) + 1 + 255) & ~size_t(255);
-  const auto aligned = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
-  if (flags <= kFlagLines && cone_takes(mapsz, vnum) && aligned(map->occ) && aligned(map->cnt) &&
-      aligned(map->hit)) {
+  if (flags <= kFlagLines && cone_takes(mapsz, vnum) && aligned(map->occ, 16) &&
+      aligned(map->cnt, 16) && aligned(map->hit, 16)) {
     p.dirty = base;
     p.hot = base + flags;
     if ((e = cudaMemsetAsync(base, 0, 2 * flags, s)) == cudaSuccess) {
@@ -200,7 +223,7 @@ int cublox_integrate_noalloc(const cublox_map_view *map, const float *xyz_soa, i
     if (e != cudaSuccess)
       return noalloc_fail(CUBLOX_ERR_CUDA, std::string("cublox_integrate_noalloc: raycast: ") +
                                                cudaGetErrorString(e));
-    return fold(map, p, 2, static_cast<int>(lines), s);
+    return fold(map, p, 0, p.vnum, 2, static_cast<int>(lines), s);
   }
 
   BinnedScratch b{reinterpret_cast<int *>(base), reinterpret_cast<int *>(base + kOffHist),
@@ -212,7 +235,7 @@ int cublox_integrate_noalloc(const cublox_map_view *map, const float *xyz_soa, i
   if (e != cudaSuccess)
     return noalloc_fail(CUBLOX_ERR_CUDA, std::string("cublox_integrate_noalloc: raycast: ") +
                                              cudaGetErrorString(e));
-  return fold(map, p, 1, 0, s);
+  return fold_sweep(map, p, s);
 }
 
 }  // extern "C"

@@ -483,8 +483,9 @@ int cublox_server_scratch_bytes(const cublox_server_config *cfg, uint64_t *bytes
  * the map view's occ / cnt / hit arrays (voxel_num elements each, in the
  * ring-buffer hash order; cnt and hit must be zero before the first call
  * and are left zero by every call) and the points, a device array of n x,
- * then n y, then n z.  The call integrates one scan exactly as
- * cublox_grid_update does for the same window origin (there is no
+ * then n y, then n z.  Arrays on 16-byte boundaries are the fast case; any
+ * that starts off a 4-byte boundary is refused (CUBLOX_ERR_INVALID).  The
+ * call integrates one scan exactly as cublox_grid_update does for the same window origin (there is no
  * first-run origin snap: origin_index is used as given), enqueues on
  * `stream` (a cudaStream_t, NULL for the default stream) and returns.
  *
