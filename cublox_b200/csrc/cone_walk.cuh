@@ -135,7 +135,8 @@ __device__ __forceinline__ void cone_order(const RayParams &p, int start, int co
       it.y[e] = y;
       it.z[e] = z;
       key[r] = (cone_place(x - p.o[0], y - p.o[1], z - p.o[2]) << 10) | e;
-      finite = finite || isfinite(x + y + z);  // a sum out of range: no finite length
+      // coordinate by coordinate: the sum of finite ones may be out of range
+      finite = finite || (isfinite(x) && isfinite(y) && isfinite(z));
     }
   }
   if (!__syncthreads_or(finite)) return;
