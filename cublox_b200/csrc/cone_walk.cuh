@@ -36,6 +36,7 @@ namespace cublox_b200 {
 // zeros at the table's end.
 constexpr int kBlock = 4;  // steps walked between two looks at who is left
 constexpr int kLeave = -(1 << 29);
+constexpr float kConeMaxRes = 1e25f;  // cone_walk: longer voxels are walked step by step
 constexpr int kConeTableMax = 8192;  // words of shared memory a table may take
 
 CBX_HD int64_t cone_table_words(const int map[3]) {
@@ -297,9 +298,12 @@ __device__ __forceinline__ void cone_walk(const RayParams &p, const int *table, 
     }
     // With a time that is no number (or that its first step makes one, from
     // -inf), or with none finite, ray_step's rule may pick an axis that the
-    // ray does not move on: walked here, step by step.
+    // ray does not move on, which has no steps in the table: walked here, step
+    // by step.  So is a map whose steps are so long that adding them up could
+    // leave no time finite (below kConeMaxRes the time of a ray's longest axis
+    // grows by less than 2e25 a step, in up to 2^33 steps).
     const float inf = inf_f();
-    if (!(w.tM[0] > -inf) || !(w.tM[1] > -inf) || !(w.tM[2] > -inf) ||
+    if (!(p.res < kConeMaxRes) || !(w.tM[0] > -inf) || !(w.tM[1] > -inf) || !(w.tM[2] > -inf) ||
         !(fminf(w.tM[0], fminf(w.tM[1], w.tM[2])) < inf)) {
       int last = -1;
       while (k < w.max_steps && !at_end(w) && !left_for_good(w, p)) {

@@ -38,3 +38,13 @@ def test_points_whose_coordinates_add_up_to_infinity(n):
     """An item all of whose points have x + y + z out of range, 5 m above a
     sensor as far out: rays like any other."""
     _same((4, 4, 4), 1e30, 100.0, [2e38, 2e38, 0.0], [[2e38, 2e38, 5.0]] * n)
+
+
+@pytest.mark.parametrize("res,max_range", [(2.476250399962677e38, 3e38), (1e25, 3e38), (9e24, 3e38)])
+@pytest.mark.parametrize("n", [1, 65])
+def test_times_that_run_out_of_range(n, res, max_range):
+    """A ray that steps past its endpoint on voxels as long as the float range:
+    no axis has a finite time left, and the rule picks one that the ray does not
+    move on.  From 1e25 m on, maps are walked step by step."""
+    s = [-2.83568231e18, 1.00390983e9, 0.0]
+    _same((3, 3, 3), res, max_range, s, [[0.0, -0.0, 0.0]] * n)
