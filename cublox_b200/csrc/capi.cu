@@ -1397,10 +1397,12 @@ static int ensure_pinned(void **p, size_t *have, size_t bytes) {
   return CUBLOX_OK;
 }
 
-// Finds the fetch's samples: sc->hoff[0 .. nq] are the queries' offsets, and,
-// with `write`, the samples are in sc->fpos and sc->fstate when it returns.
+// Finds the fetch's samples: sc->hoff[0 .. nq] are the queries' offsets, *total
+// the last of them, and, with `write`, the samples are in sc->fpos and
+// sc->fstate when it returns.  What an earlier fetch_begin left there is gone.
 static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int nq, float radius,
-                     int filter, int max_results, bool write, FetchScratch *sc) {
+                     int filter, int max_results, bool write, FetchScratch *sc, int64_t *total) {
+  *total = 0;
   if (!g || (nq > 0 && !centers)) return fail(CUBLOX_ERR_INVALID, "fetch: null argument");
   if (!sc) sc = &g->fs;
   if (filter < -1 || filter > 2) return fail(CUBLOX_ERR_INVALID, "fetch: bad filter");
@@ -1410,10 +1412,7 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
   if (rc) return rc;
   long long *off = static_cast<long long *>(sc->hoff);
   off[0] = 0;
-  if (nq == 0) {
-    sc->pending = 0;
-    return CUBLOX_OK;
-  }
+  if (nq == 0) return CUBLOX_OK;
   FetchParams p{};
   // tiles: the bricks' columns (at most 32, as in every layout of 32-voxel
   // bricks); in the reference's order, 8 x 4 columns
@@ -1504,10 +1503,9 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
   CK(cudaMemcpyAsync(off, p.offsets, sizeof(long long) * (static_cast<size_t>(nq) + 1),
                      cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  if (!write) return CUBLOX_OK;
-  const long long total = off[nq];
-  if (total > p.room) {
-    if ((rc = ensure_fout(sc, st, total))) return rc;
+  *total = off[nq];
+  if (write && *total > p.room) {
+    if ((rc = ensure_fout(sc, st, *total))) return rc;
     p.room = sc->fcap;
     p.out_pos = sc->fpos;
     p.out_state = sc->fstate;
@@ -1515,7 +1513,6 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
     CK_LAUNCH();
     CK(cudaStreamSynchronize(st));
   }
-  sc->pending = total;
   return CUBLOX_OK;
 }
 
@@ -1587,10 +1584,10 @@ static int copy_out(cublox_grid *g, cudaStream_t st, FetchScratch *sc,
   return CUBLOX_OK;
 }
 
-// The pending fetch's samples to host memory (null: not wanted).
-static int fetch_copy(cublox_grid *g, cudaStream_t st, FetchScratch *sc, float *out_pos,
-                      uint8_t *out_state) {
-  const size_t n = static_cast<size_t>(sc->pending);
+// The n samples that fetch_run wrote to host memory (null: not wanted).
+static int fetch_copy(cublox_grid *g, cudaStream_t st, FetchScratch *sc, int64_t samples,
+                      float *out_pos, uint8_t *out_state) {
+  const size_t n = static_cast<size_t>(samples);
   if (n == 0) return CUBLOX_OK;
   std::pair<const void *, void *> parts[2] = {{sc->fpos, out_pos}, {sc->fstate, out_state}};
   size_t bytes[2] = {12 * n, n};
@@ -1612,11 +1609,12 @@ int cublox_b200::detail::fetch_into(cublox_grid *g, cudaStream_t st, const float
                                     std::vector<int64_t> &offsets,
                                     const std::function<void *(size_t)> &room, FetchScratch *sc) {
   if (!sc) sc = &g->fs;
-  const int rc = fetch_run(g, st, centers, nq, radius, filter, max_results, true, sc);
+  int64_t total = 0;
+  const int rc = fetch_run(g, st, centers, nq, radius, filter, max_results, true, sc, &total);
   if (rc) return rc;
   const long long *off = static_cast<const long long *>(sc->hoff);
   offsets.assign(off, off + nq + 1);
-  const size_t n = static_cast<size_t>(sc->pending);
+  const size_t n = static_cast<size_t>(total);
   if (n == 0) return CUBLOX_OK;
   char *dst = static_cast<char *>(room(13 * n));
   if (!dst) return fail(CUBLOX_ERR_NOMEM, "fetch: no memory for the samples");
@@ -1665,9 +1663,9 @@ int cublox_grid_fetch_viz(cublox_grid *g, const float center[3], float radius, i
   if (!g || !center || !robot_pos || !n_out || (capacity > 0 && !out_xyzrgb))
     return fail(CUBLOX_ERR_INVALID, "fetch_viz: null argument");
   if (max_points < 0) return fail(CUBLOX_ERR_INVALID, "fetch_viz: negative max_points");
-  int rc = fetch_run(g, g->stream, center, 1, radius, filter, max_results, true, &g->fs);
+  int64_t total = 0;
+  int rc = fetch_run(g, g->stream, center, 1, radius, filter, max_results, true, &g->fs, &total);
   if (rc) return rc;
-  const int64_t total = g->fs.pending;
   if (total == 0 || max_points == 0) return CUBLOX_OK;
   const int64_t cap = std::min<int64_t>(max_points, total);
   if (capacity < cap)
@@ -1720,33 +1718,43 @@ int cublox_grid_fetch(cublox_grid *g, const float center[3], float radius,
                       uint8_t *out_state, int64_t capacity, int64_t *n_out) {
   if (n_out) *n_out = 0;
   if (!g || !center) return fail(CUBLOX_ERR_INVALID, "cublox_grid_fetch: null argument");
-  int rc = fetch_run(g, g->stream, center, 1, radius, filter, max_results, true, &g->fs);
+  int64_t kept = 0;
+  int rc = fetch_run(g, g->stream, center, 1, radius, filter, max_results, true, &g->fs, &kept);
   if (rc) return rc;
-  const int64_t kept = g->fs.pending;
   if (kept > capacity)
     return fail(CUBLOX_ERR_INVALID, "cublox_grid_fetch: capacity " + std::to_string(capacity) +
                                         " < " + std::to_string(kept) + " samples");
-  if ((rc = fetch_copy(g, g->stream, &g->fs, out_pos, out_state))) return rc;
+  if ((rc = fetch_copy(g, g->stream, &g->fs, kept, out_pos, out_state))) return rc;
   if (n_out) *n_out = kept;
   return CUBLOX_OK;
 }
 
-int cublox_grid_fetch_begin(cublox_grid *g, const float *centers, int n_centers, float radius,
-                            int filter, int max_results, int64_t *out_offsets) {
-  if (!out_offsets) return fail(CUBLOX_ERR_INVALID, "fetch_begin: null offsets");
+// A fetch of many centres on the grid's own scratch, with its offsets copied out.
+static int fetch_many(cublox_grid *g, const float *centers, int n_centers, float radius, int filter,
+                      int max_results, int64_t *out_offsets, int64_t *total) {
   const int rc = fetch_run(g, g ? g->stream : nullptr, centers, n_centers, radius, filter,
-                           max_results, true, nullptr);
+                           max_results, true, nullptr, total);
   if (rc) return rc;
   const long long *off = static_cast<const long long *>(g->fs.hoff);
   std::copy(off, off + std::max(n_centers, 0) + 1, out_offsets);
   return CUBLOX_OK;
 }
 
+int cublox_grid_fetch_begin(cublox_grid *g, const float *centers, int n_centers, float radius,
+                            int filter, int max_results, int64_t *out_offsets) {
+  if (!out_offsets) return fail(CUBLOX_ERR_INVALID, "fetch_begin: null offsets");
+  int64_t total = 0;
+  const int rc =
+      fetch_many(g, centers, n_centers, radius, filter, max_results, out_offsets, &total);
+  if (!rc) g->fs.pending = total;
+  return rc;
+}
+
 int cublox_grid_fetch_read(cublox_grid *g, float *out_pos, uint8_t *out_state, int64_t n) {
   if (!g) return fail(CUBLOX_ERR_INVALID, "null grid");
   if (g->fs.pending < 0 || n != g->fs.pending)
     return fail(CUBLOX_ERR_INVALID, "fetch_read: not the samples of the last fetch_begin");
-  return fetch_copy(g, g->stream, &g->fs, out_pos, out_state);
+  return fetch_copy(g, g->stream, &g->fs, n, out_pos, out_state);
 }
 
 int cublox_grid_fetch_batch(cublox_grid *g, const float *centers,
@@ -1755,21 +1763,23 @@ int cublox_grid_fetch_batch(cublox_grid *g, const float *centers,
                             float *out_pos, uint8_t *out_state,
                             int64_t capacity) {
   if (!out_offsets) return fail(CUBLOX_ERR_INVALID, "fetch_batch: null offsets");
+  int64_t total = 0;
   const int rc =
-      cublox_grid_fetch_begin(g, centers, n_centers, radius, filter, max_results, out_offsets);
+      fetch_many(g, centers, n_centers, radius, filter, max_results, out_offsets, &total);
   if (rc) return rc;
-  if (g->fs.pending > capacity)
+  if (total > capacity)
     return fail(CUBLOX_ERR_INVALID, "fetch: output capacity " + std::to_string(capacity) + " < " +
-                                        std::to_string(g->fs.pending) + " samples");
-  return fetch_copy(g, g->stream, &g->fs, out_pos, out_state);
+                                        std::to_string(total) + " samples");
+  return fetch_copy(g, g->stream, &g->fs, total, out_pos, out_state);
 }
 
 int cublox_grid_fetch_counts(cublox_grid *g, const float *centers,
                              int n_centers, float radius, int filter,
                              int max_results, int64_t *out_counts) {
   if (!out_counts) return fail(CUBLOX_ERR_INVALID, "fetch_counts: null output");
+  int64_t total = 0;
   const int rc = fetch_run(g, g ? g->stream : nullptr, centers, n_centers, radius, filter,
-                           max_results, false, nullptr);
+                           max_results, false, nullptr, &total);
   if (rc) return rc;
   const long long *off = static_cast<const long long *>(g->fs.hoff);
   for (int i = 0; i < n_centers; ++i) out_counts[i] = off[i + 1] - off[i];

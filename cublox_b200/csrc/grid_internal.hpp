@@ -21,7 +21,7 @@ struct FetchScratch {
   float *fpos = nullptr;
   uint8_t *fstate = nullptr;
   int64_t fcap = 0;
-  int64_t pending = -1;  // samples of the last fetch, in fpos and fstate (-1: none)
+  int64_t pending = -1;  // samples of a fetch_begin, still in fpos and fstate (-1: none)
   void *hoff = nullptr;  // pinned: the queries' offsets
   size_t hoff_bytes = 0;
   void *hcopy = nullptr;  // pinned: samples on their way to pageable memory

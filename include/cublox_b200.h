@@ -216,8 +216,10 @@ int cublox_grid_fetch_batch(cublox_grid *g, const float *centers,
                             int64_t capacity);
 /* The same in two calls, for callers that size their outputs by the number
  * of samples: begin finds them (out_offsets as above, n_centers + 1 entries)
- * and keeps them on the device; read copies them out, n = out_offsets[last].
- * read refuses any other n, and a grid on which another fetch was made since.
+ * and keeps them on the device; read copies them out, n = out_offsets[last],
+ * as often as it is called.  read gives the samples of the grid's last begin:
+ * it refuses any other n, and a grid on which fetch, fetch_batch, fetch_viz
+ * or fetch_counts was called since that begin, or no begin at all.
  * No counterpart in the reference.                                          */
 int cublox_grid_fetch_begin(cublox_grid *g, const float *centers, int n_centers, float radius,
                             int filter, int max_results, int64_t *out_offsets);
