@@ -338,7 +338,7 @@ class OccupancyGrid:
 
         Returns (positions (n, 3) float32, states (n,) uint8), ordered by
         ascending (x, y, z) global voxel index."""
-        _, pos, st = self._fetch([center], radius, state_filter, max_results, "fetchOccupancyAround")
+        _, pos, st = self._fetch(list(_f3(center)), radius, state_filter, max_results, "fetchOccupancyAround")
         return pos, st
 
     def fetch_batch(self, centers, radius: float, state_filter=None, max_results: int = 0):
