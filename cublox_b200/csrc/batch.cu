@@ -752,8 +752,10 @@ struct cublox_batch {
   bool graphs = false;
   bool host_read = true;  // the walk reads host points in place (CUBLOX_BATCH_OPT_HOST_READ)
   int fold_variant = 0;
-  cudaGraphExec_t graph = nullptr;
-  int graph_shape = -1;
+  // the captured launches: [0] of the batch's shape, [1] of kWideShape in its
+  // place, so that updates with and without a wide map may take turns
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  int graph_shape[2] = {-1, -1};
   // timing
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   bool timed = false;
@@ -781,7 +783,7 @@ int ensure_dev(void **p, size_t bytes) {
   return CUBLOX_OK;
 }
 
-void drop_graph(cublox_batch *b);
+void drop_graphs(cublox_batch *b);
 
 int ensure_capacity(cublox_batch *b, int n_maps, int n_witems, int n_fitems) {
   if (n_maps > b->maps_cap || n_witems > b->witems_cap || n_fitems > b->fitems_cap) {
@@ -800,17 +802,13 @@ int ensure_capacity(cublox_batch *b, int n_maps, int n_witems, int n_fitems) {
         (rc = ensure_pinned(reinterpret_cast<void **>(&b->h_fitems), sizeof(FoldItem) * fc))) {
       // some buffers are gone: the next update sizes them all again
       b->maps_cap = b->witems_cap = b->fitems_cap = 0;
-      drop_graph(b);
+      drop_graphs(b);
       return rc;
     }
     b->maps_cap = mc;
     b->witems_cap = wc;
     b->fitems_cap = fc;
-    if (b->graph) {  // pointers changed: recapture
-      cudaGraphExecDestroy(b->graph);
-      b->graph = nullptr;
-      b->graph_shape = -1;
-    }
+    drop_graphs(b);  // pointers changed: recapture
   }
   return CUBLOX_OK;
 }
@@ -873,10 +871,15 @@ cudaError_t enqueue_step(cublox_batch *b, int shape, const char **what) {
   return cudaSuccess;
 }
 
-void drop_graph(cublox_batch *b) {
-  if (b->graph) cudaGraphExecDestroy(b->graph);
-  b->graph = nullptr;
-  b->graph_shape = -1;
+void drop_graph(cublox_batch *b, int which) {
+  if (b->graph[which]) cudaGraphExecDestroy(b->graph[which]);
+  b->graph[which] = nullptr;
+  b->graph_shape[which] = -1;
+}
+
+void drop_graphs(cublox_batch *b) {
+  drop_graph(b, 0);
+  drop_graph(b, 1);
 }
 
 }  // namespace
@@ -915,7 +918,7 @@ int cublox_batch_destroy(cublox_batch *b) {
   if (!b) return CUBLOX_OK;
   cudaStreamSynchronize(b->stream);
   for (cublox_grid *g : b->grids) cublox_grid_destroy(g);
-  if (b->graph) cudaGraphExecDestroy(b->graph);
+  drop_graphs(b);
   cublox_b200::detail::dfree(b->d_maps);
   cublox_b200::detail::dfree(b->d_witems);
   cublox_b200::detail::dfree(b->d_fitems);
@@ -984,7 +987,7 @@ int cublox_batch_set_option(cublox_batch *b, int key, int value) {
     case CUBLOX_BATCH_OPT_FOLD:
       if (value < 0 || value > 2) break;
       b->fold_variant = value;
-      drop_graph(b);
+      drop_graphs(b);
       return CUBLOX_OK;
     default:
       break;
@@ -1032,9 +1035,10 @@ int cublox_batch_update(cublox_batch *b, int n, cublox_grid *const *grids, const
   const bool tuning = b->autotune && b->tune_step < kNumCandidates * b->tune_rounds;
   const int cand = tuning ? (b->tune_step / b->tune_rounds) % kNumCandidates : -1;
   int active_shape = tuning ? kCandidates[cand].shape : b->shape;
+  bool wide = false;
   if (kShapes[active_shape].cone)
-    for (int i = 0; i < n; ++i)
-      if (!cone_takes(grids[i]->map, grids[i]->nalloc)) active_shape = kWideShape;
+    for (int i = 0; i < n; ++i) wide = wide || !cone_takes(grids[i]->map, grids[i]->nalloc);
+  if (wide) active_shape = kWideShape;
   const int active_layout = tuning ? kCandidates[cand].layout : b->layout;
   // the grids' voxel layout (moved between scans, on the batch's stream)
   for (int i = 0; i < n; ++i) {
@@ -1174,8 +1178,9 @@ int cublox_batch_update(cublox_batch *b, int n, cublox_grid *const *grids, const
   const bool timed_before = b->timed;
   if (tuning) b->timed = true;
   if (b->graphs && !tuning && !b->timed) {
-    if (!b->graph || b->graph_shape != active_shape) {
-      drop_graph(b);
+    cudaGraphExec_t &graph = b->graph[wide];
+    if (!graph || b->graph_shape[wide] != active_shape) {
+      drop_graph(b, wide);
       cudaGraph_t gr;
       if ((e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
         return cuda_fail(e, "batch graph capture", __LINE__);
@@ -1185,13 +1190,13 @@ int cublox_batch_update(cublox_batch *b, int n, cublox_grid *const *grids, const
       if (le != cudaSuccess)
         return cuda_fail(le, (std::string("batch graph capture: ") + what).c_str(), __LINE__);
       if (e != cudaSuccess) return cuda_fail(e, "batch graph end capture", __LINE__);
-      e = cudaGraphInstantiate(&b->graph, gr, 0);
+      e = cudaGraphInstantiate(&graph, gr, 0);
       detail::count(detail::kGraphBuilds);
       cudaGraphDestroy(gr);
       if (e != cudaSuccess) return cuda_fail(e, "batch graph instantiate", __LINE__);
-      b->graph_shape = active_shape;
+      b->graph_shape[wide] = active_shape;
     }
-    if ((e = cudaGraphLaunch(b->graph, b->stream)) != cudaSuccess)
+    if ((e = cudaGraphLaunch(graph, b->stream)) != cudaSuccess)
       return cuda_fail(e, "batch graph launch", __LINE__);
   } else {
     const char *what = "";
