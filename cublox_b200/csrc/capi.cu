@@ -610,13 +610,46 @@ static int ensure_stage(cublox_grid *g, int n) {
   return CUBLOX_OK;
 }
 
-// The default walk goes in direction order (cone_walk.cuh), about twice as
-// fast as the split walk at every size measured (raycast_cone.cu), unless the
-// map is too wide for it or an option of the split walk was set.
-static bool walks_cones(const cublox_grid *g) {
+// Whether the walk in direction order is the faster one for a scan of n rays
+// from `sensor`.  It takes a ray's steps one after another, so that its time is
+// at least that of the longest ray the map and the range allow: `chain` steps,
+// about 0.1 us each.  The split walk cuts rays every 64 steps, but plans each
+// ray and adds every voxel by a request of its own.  How many voxels there are
+// is estimated from `mean`, the steps of a level ray to the window's sides over
+// all azimuths: in a corridor few rays are long.  The line was fitted to both
+// walks' times of 84 scans, and takes the faster one, or one within 4 %, for
+// each.  Some of them in direction order / split, us, by half sizes and rays:
+// 350 x 350 x 75, 2,000 109 / 128 and 65,536 216 / 362; 1000 x 500 x 30, 2,000
+// 183 / 140, 16,384 206 / 210, 65,536 261 / 393; 1990 x 20 x 20, 16,384 220 /
+// 128, 65,536 236 / 154, 262,144 272 / 348.  No scan whose chain is below 710
+// steps is split.
+static bool cone_pays(const cublox_grid *g, int n, const float sensor[3]) {
+  // voxels a ray can cross, a number also where the range is none
+  const float range = g->max_range * g->res_inv;
+  const float reach = range < 1e6f ? std::max(range, 0.0f) : 1e6f;
+  float far[3], near[3];
+  for (int a = 0; a < 3; ++a) {
+    const int64_t off = static_cast<int64_t>(host_p2g(sensor[a], g->res_inv, g->ctr)) - g->origin_i[a];
+    const int half = g->half[a];
+    far[a] = static_cast<float>(half + std::min<int64_t>(std::abs(off), half));
+    near[a] = std::max(1.0f, std::min(static_cast<float>(half), reach));
+  }
+  // a ray's steps are at most sqrt(3) times its length; few go far up or down
+  const float level = far[0] + far[1];
+  const float chain = std::min(level + std::min(far[2], level), 1.7321f * reach + 4.0f);
+  const float a = std::max(near[0], near[1]), b = std::min(near[0], near[1]);
+  const float t = std::atan2(b, a);  // azimuth of the window's corner
+  const float mean = 0.6366f * (a * (t - std::log(std::cos(t))) +
+                                b * (1.5708f - t - std::log(std::sin(t))));
+  return chain <= 710.0f + 0.17f * mean + 4.7e-3f * n + 41e-6f * n * mean;
+}
+
+// The default walk goes in direction order (cone_walk.cuh), unless the map is
+// too wide for it, an option of the split walk was set, or that is faster.
+static bool walks_cones(const cublox_grid *g, int n, const float sensor[3]) {
   return g->opt_raycast == 2 && g->opt_cube == 32 && !g->opt_flat && !g->opt_sort &&
          g->opt_seg == 64 && g->opt_block == 512 && !g->opt_contig &&
-         cone_takes(g->map, g->nalloc);
+         cone_takes(g->map, g->nalloc) && cone_pays(g, n, sensor);
 }
 
 // Launch raycast (+ fold unless count_only) on a device cloud.
@@ -669,7 +702,7 @@ static int integrate(cublox_grid *g, const float *dx, const float *dy,
     g->bin_cap = n;
   }
   tmark(g, 0, 0);
-  const bool cone = walks_cones(g);
+  const bool cone = walks_cones(g, n, sensor);
   const bool split = g->opt_raycast == 2 && !cone;
   if (split && p.stride != 1) {
     // the split walk reads SoA: gather an AoS cloud first
@@ -933,7 +966,8 @@ static int update_impl(cublox_grid *g, const float *x, const float *y,
   CK(cudaEventSynchronize(g->stage_ev[s]));
   float *h = g->h_stage[s];
   const size_t nb = sizeof(float) * static_cast<size_t>(n);
-  const bool as_is = xyz && layout == CUBLOX_LAYOUT_AOS && walks_cones(g);  // reads any stride
+  // that walk reads any stride
+  const bool as_is = xyz && layout == CUBLOX_LAYOUT_AOS && walks_cones(g, n, sensor);
   if (as_is) {
     std::memcpy(h, xyz, 3 * nb);
   } else if (xyz && layout == CUBLOX_LAYOUT_AOS) {
