@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <deque>
 #include <limits>
 #include <functional>
 #include <string>
@@ -1376,11 +1377,15 @@ QueryBox plan_query(const cublox_grid *g, const float c[3], float radius) {
 }
 }  // namespace
 
-// Fetch scratch grows geometrically: a reallocation frees memory, which
-// waits for the whole device.
+// Bytes of a grid's query block, and of one where that is not to be had.
+constexpr size_t kFetchBlock = static_cast<size_t>(64) << 20;
+constexpr size_t kFetchLeast = static_cast<size_t>(1) << 20;
+
+// Fetch scratch grows geometrically (the query block up to its bound): a
+// reallocation frees memory, which waits for the whole device.
 static int ensure_fq(FetchScratch *sc, cudaStream_t st, size_t bytes) {
   if (bytes <= sc->fq_bytes) return CUBLOX_OK;
-  bytes = std::max({bytes, 2 * sc->fq_bytes, static_cast<size_t>(4) << 10});
+  bytes = std::max({bytes, std::min(2 * sc->fq_bytes, kFetchBlock), static_cast<size_t>(4) << 10});
   CK(cudaStreamSynchronize(st));
   cublox_b200::detail::dfree(sc->fq);
   sc->fq = nullptr;
@@ -1410,19 +1415,134 @@ static int ensure_fout(FetchScratch *sc, cudaStream_t st, int64_t n) {
   return CUBLOX_OK;
 }
 
-// The query block of a fetch in its scratch: queries | units | columns |
-// level masks | rows | kept | offsets.
-struct FetchBlock {
-  size_t units, col, mask, row, kept, offsets, bytes;
-  FetchBlock(size_t nq, size_t nu, size_t cols, size_t words, size_t rows) {
-    auto al = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
-    units = al(sizeof(FetchQuery) * nq);
-    col = units + al(sizeof(int2) * nu);
-    mask = col + al(sizeof(int) * cols);
-    row = mask + al(sizeof(uint32_t) * words);
-    kept = row + al(sizeof(int) * rows);
-    offsets = kept + al(sizeof(int) * nq);
-    bytes = offsets + al(sizeof(long long) * (nq + 1));
+static size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
+
+// What one launch of a fetch's kernels takes of the query block: its queries |
+// units | rows | columns | level masks.
+struct FetchSizes {
+  size_t queries = 0, units = 0, rows = 0, columns = 0, words = 0;
+  size_t at_units() const { return align256(sizeof(FetchQuery) * queries); }
+  size_t at_rows() const { return at_units() + align256(sizeof(int2) * units); }
+  size_t at_columns() const { return at_rows() + align256(sizeof(int) * rows); }
+  size_t at_masks() const { return at_columns() + align256(sizeof(int) * columns); }
+  size_t bytes() const { return at_masks() + align256(sizeof(uint32_t) * words); }
+};
+
+// Consecutive queries of a fetch that share a launch, or a part of the units of
+// one query that is too large for that.
+struct FetchGroup {
+  FetchSizes size;
+  size_t q0 = 0, nq = 0;                  // queries
+  const FetchQuery *queries = nullptr;    // their descriptors
+  size_t u0 = 0, nu = 0;                  // units
+  int most = 1;                           // tiles along y, of any query
+  size_t parts = 1;                       // groups of the same query from here on
+};
+
+// A fetch cut into groups of at most `limit` bytes of the query block each
+// (usually one), so that scratch does not grow with the columns and levels of
+// its boxes.  A query that is alone in a group and does not fit goes without
+// level masks (its samples are found twice), then in parts: counted part by
+// part, and, with its rows known, counted once more part by part and written.
+struct FetchPlan {
+  std::vector<FetchQuery> queries;
+  std::vector<int2> units;
+  std::vector<FetchGroup> groups;
+  std::deque<FetchQuery> parts;  // descriptors of queries in parts
+  size_t bytes = 0;              // the largest group's
+  const int row_bits;
+  const bool masks;
+
+  FetchPlan(size_t n, int row_bits_, bool masks_) : row_bits(row_bits_), masks(masks_) {
+    queries.reserve(n);
+  }
+
+  // One more query, into the one group that all of them would make.
+  void push(FetchQuery &q) {
+    add(&all_, queries.size(), q, with(all_.size, q, static_cast<size_t>(q.nt[0]), masks), 0,
+        static_cast<size_t>(q.nt[0]));
+    queries.push_back(q);
+  }
+
+  void cut(size_t limit) {
+    groups.clear();
+    parts.clear();
+    bytes = 0;
+    if (!cut_ && all_.size.bytes() <= limit) {
+      groups.push_back(all_);
+      groups[0].queries = queries.data();
+      bytes = all_.size.bytes();
+      return;
+    }
+    cut_ = true;  // the places that push gave are overwritten
+    units.clear();
+    FetchGroup g;
+    for (size_t i = 0; i < queries.size(); ++i) {
+      FetchQuery &q = queries[i];
+      const size_t nu = static_cast<size_t>(q.nt[0]);
+      FetchSizes s = with(g.size, q, nu, masks);
+      if (g.nq && s.bytes() > limit) {
+        close(&g);
+        s = with(g.size, q, nu, masks);
+      }
+      if (s.bytes() <= limit) {
+        add(&g, i, q, s, 0, nu);
+        continue;
+      }
+      s = with(FetchSizes{}, q, nu, false);
+      size_t step = nu;
+      if (s.bytes() > limit) {  // the same places in each part
+        const size_t fixed = with(FetchSizes{}, q, 0, false).bytes() + 512;  // and two roundings
+        const size_t per = sizeof(int2) + sizeof(int) * (static_cast<size_t>(q.n[1]) << row_bits);
+        step = std::max<size_t>(1, std::min(limit > fixed ? (limit - fixed) / per : 0, nu));
+        s = with(FetchSizes{}, q, step, false);
+      }
+      for (size_t first = 0; first < nu; first += step) {
+        parts.push_back(q);
+        parts.back().u0 = static_cast<int>(first);
+        add(&g, i, parts.back(), s, first, std::min(step, nu - first));
+        g.parts = (nu - first + step - 1) / step;
+        close(&g);
+      }
+    }
+    if (g.nq) close(&g);
+  }
+
+ private:
+  FetchGroup all_;
+  bool cut_ = false;
+
+  // The sizes of a group with n_units units of q added.
+  FetchSizes with(FetchSizes s, const FetchQuery &q, size_t n_units, bool masked) const {
+    const size_t columns = n_units * (static_cast<size_t>(q.n[1]) << row_bits);
+    ++s.queries;
+    s.units += n_units;
+    s.rows += static_cast<size_t>(q.n[0]);
+    s.columns += columns;
+    if (masked) s.words += columns * ((static_cast<size_t>(q.n[2]) + 31) / 32);
+    return s;
+  }
+  // Adds units first, ... of q, which is (a part of) query i, to the group.
+  void add(FetchGroup *g, size_t i, FetchQuery &q, const FetchSizes &s, size_t first, size_t n) {
+    if (!g->nq) {
+      g->q0 = i;
+      g->queries = &q;
+      g->u0 = units.size();
+    }
+    q.row0 = static_cast<long long>(g->size.rows);
+    q.col0 = static_cast<long long>(g->size.columns);
+    q.mask0 = static_cast<long long>(g->size.words);
+    g->size = s;
+    for (size_t t = first; t < first + n; ++t)
+      units.push_back(make_int2(static_cast<int>(g->nq), static_cast<int>(t)));
+    g->most = std::max(g->most, q.nt[1]);
+    ++g->nq;
+    g->nu += n;
+  }
+  void close(FetchGroup *g) {
+    bytes = std::max(bytes, g->size.bytes());
+    groups.push_back(*g);
+    *g = FetchGroup{};
   }
 };
 
@@ -1462,58 +1582,64 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
   // bricks); in the reference's order, 8 x 4 columns
   p.lt[0] = g->lay_code == 0 ? 3 : g->lay.lb[0];
   p.lt[1] = g->lay_code == 0 ? 2 : g->lay.lb[1];
-  std::vector<FetchQuery> queries(nq);
-  std::vector<int2> units;
-  int64_t cols = 0, words = 0, rows = 0;
-  int most = 1;
+  int low_slot[2];  // of the window's first voxel; a box lies in the window
+  for (int a = 0; a < 2; ++a)
+    low_slot[a] = global_to_local(g->origin_i[a] - g->half[a], g->map[a], g->half[a]) + g->half[a];
+  FetchPlan plan(static_cast<size_t>(nq), p.lt[0], write && filter >= 0);
   for (int i = 0; i < nq; ++i) {
     const float *c = centers + 3 * static_cast<size_t>(i);
     const QueryBox b = plan_query(g, c, radius);
-    FetchQuery &q = queries[i];
-    q = FetchQuery{};
+    FetchQuery q{};
     for (int a = 0; a < 3; ++a) {
       q.c[a] = c[a];
       q.g0[a] = b.box[2 * a];
       q.n[a] = b.box[2 * a + 1] - b.box[2 * a] + 1;
     }
     q.r2 = b.r2;
-    q.row0 = rows;
-    q.col0 = cols;
-    q.mask0 = words;
     if (q.n[0] <= 0 || q.n[1] <= 0 || q.n[2] <= 0) {
       q.n[0] = q.n[1] = q.n[2] = 0;
+      plan.push(q);
       continue;
     }
     for (int a = 0; a < 2; ++a) {
-      const int m = g->map[a], h = g->half[a], tiles = (m + (1 << p.lt[a]) - 1) >> p.lt[a];
-      const int first = global_to_local(q.g0[a], m, h) + h;
-      const int last = global_to_local(q.g0[a] + q.n[a] - 1, m, h) + h;
+      const int m = g->map[a], tiles = (m + (1 << p.lt[a]) - 1) >> p.lt[a];
+      int first = low_slot[a] + (q.g0[a] - (g->origin_i[a] - g->half[a]));
+      if (first >= m) first -= m;
+      int last = first + q.n[a] - 1;
+      if (last >= m) last -= m;
       q.t0[a] = first >> p.lt[a];
       // around the ring where the box wraps; its two ends may share a tile
       const int span = (last >> p.lt[a]) - q.t0[a] + 1 + (last < first ? tiles : 0);
       q.nt[a] = std::min(span, tiles);
     }
-    for (int t = 0; t < q.nt[0]; ++t) units.push_back(make_int2(i, t));
-    most = std::max(most, q.nt[1]);
-    rows += q.n[0];
-    cols += static_cast<int64_t>(q.n[0]) * q.n[1];
-    if (filter >= 0) words += static_cast<int64_t>(q.n[0]) * q.n[1] * ((q.n[2] + 31) / 32);
+    plan.push(q);
   }
-  const int nu = static_cast<int>(units.size());
-  const FetchBlock blk(static_cast<size_t>(nq), units.size(), static_cast<size_t>(cols),
-                       static_cast<size_t>(words), static_cast<size_t>(rows));
-  if ((rc = ensure_fq(sc, st, blk.bytes))) return rc;
+  // the block: samples kept per query | offsets | the current group
+  const size_t at_offsets = align256(sizeof(int) * nq);
+  const size_t at_group = at_offsets + align256(sizeof(long long) * (static_cast<size_t>(nq) + 1));
+  const size_t least = kFetchLeast / 2;
+  const size_t bound = sc->fq_limit ? sc->fq_limit : kFetchBlock;
+  const size_t limit = std::max(bound, at_group + least) - at_group;
+  plan.cut(limit);
+  // A server's block is small, and its outputs mostly empty: a fetch of several
+  // groups has them in the second half of the outputs instead, and the samples
+  // in the first, as long as they fit.
+  const size_t half = align256(sizeof(float) * 3 * static_cast<size_t>(sc->fcap) / 2);
+  const size_t upper = sizeof(float) * 3 * static_cast<size_t>(sc->fcap) - half;
+  bool lent = sc->fq_limit && plan.groups.size() > 1 && upper > limit;
+  if (lent) {
+    plan.cut(upper);
+    lent = plan.bytes <= upper;
+    if (!lent) plan.cut(limit);
+  }
+  rc = ensure_fq(sc, st, at_group + (lent ? 0 : plan.bytes));
+  if (rc == CUBLOX_ERR_NOMEM && bound > kFetchLeast) {
+    plan.cut(least);
+    rc = ensure_fq(sc, st, at_group + plan.bytes);
+  }
+  if (rc) return rc;
   char *base = static_cast<char *>(sc->fq);
-  CK(cudaMemcpyAsync(base, queries.data(), sizeof(FetchQuery) * nq, cudaMemcpyHostToDevice, st));
-  if (nu > 0)
-    CK(cudaMemcpyAsync(base + blk.units, units.data(), sizeof(int2) * nu, cudaMemcpyHostToDevice,
-                       st));
   p.occ = g->d_occ;
-  p.queries = reinterpret_cast<const FetchQuery *>(base);
-  p.nq = nq;
-  p.units = reinterpret_cast<const int2 *>(base + blk.units);
-  p.nu = nu;
-  p.most_tiles = most;
   for (int a = 0; a < 3; ++a) {
     p.win[a] = g->origin_i[a];
     p.half[a] = g->half[a];
@@ -1528,33 +1654,80 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
   p.filter = filter;
   p.cap = max_results > 0 ? max_results : 500000;  // OccupancyGrid.cpp:292
   p.lay = g->lay;
-  p.col = reinterpret_cast<int *>(base + blk.col);
-  p.mask = write && filter >= 0 ? reinterpret_cast<uint32_t *>(base + blk.mask) : nullptr;
-  p.row = reinterpret_cast<int *>(base + blk.row);
-  p.kept = reinterpret_cast<int *>(base + blk.kept);
-  p.offsets = reinterpret_cast<long long *>(base + blk.offsets);
-  launch_fetch_count(p, st);
-  CK_LAUNCH();
+  int sms = 148;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device) != cudaSuccess)
+    cudaGetLastError();
+  p.ctas = 8 * sms;
+  // A group's descriptors, and what its kernels are told.
+  const auto load = [&](const FetchGroup &gr) {
+    char *area = lent ? reinterpret_cast<char *>(sc->fpos) + half : base + at_group;
+    p.queries = reinterpret_cast<const FetchQuery *>(area);
+    p.nq = static_cast<int>(gr.nq);
+    p.units = reinterpret_cast<const int2 *>(area + gr.size.at_units());
+    p.nu = static_cast<int>(gr.nu);
+    p.most_tiles = gr.most;
+    p.row = reinterpret_cast<int *>(area + gr.size.at_rows());
+    p.col = reinterpret_cast<int *>(area + gr.size.at_columns());
+    p.mask = gr.size.words ? reinterpret_cast<uint32_t *>(area + gr.size.at_masks()) : nullptr;
+    p.kept = reinterpret_cast<int *>(base) + gr.q0;
+    p.offsets = reinterpret_cast<long long *>(base + at_offsets) + gr.q0;
+    p.first = gr.q0 == 0;
+    cudaError_t e = cudaMemcpyAsync(area, gr.queries, sizeof(FetchQuery) * gr.nq,
+                                    cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && gr.nu)
+      e = cudaMemcpyAsync(area + gr.size.at_units(), plan.units.data() + gr.u0,
+                          sizeof(int2) * gr.nu, cudaMemcpyHostToDevice, st);
+    return e;
+  };
+  // Counts every group and, where the outputs may have room, writes it.
+  const auto run = [&](bool writes) {
+    for (size_t i = 0, parts; i < plan.groups.size(); i += parts) {
+      parts = plan.groups[i].parts;
+      p.rows_done = 0;
+      for (size_t k = i; k < i + parts; ++k) {
+        CK(load(plan.groups[k]));
+        launch_fetch_count(p, st);
+      }
+      launch_fetch_offsets(p, st);
+      p.rows_done = 1;
+      for (size_t k = i; writes && k < i + parts; ++k) {
+        if (parts > 1) {
+          CK(load(plan.groups[k]));
+          launch_fetch_count(p, st);
+        }
+        launch_fetch_write(p, st);
+      }
+      CK_LAUNCH();
+    }
+    return CUBLOX_OK;
+  };
   // The samples are written without waiting for their number where the
   // outputs of earlier fetches have room for them.
-  p.room = sc->fcap;
+  p.room = lent ? static_cast<int64_t>(half / (sizeof(float) * 3)) : sc->fcap;
   p.out_pos = sc->fpos;
   p.out_state = sc->fstate;
-  if (write && p.room > 0) {
-    launch_fetch_write(p, st);
-    CK_LAUNCH();
-  }
-  CK(cudaMemcpyAsync(off, p.offsets, sizeof(long long) * (static_cast<size_t>(nq) + 1),
+  if ((rc = run(write && p.room > 0))) return rc;
+  CK(cudaMemcpyAsync(off, base + at_offsets, sizeof(long long) * (static_cast<size_t>(nq) + 1),
                      cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   *total = off[nq];
   if (write && *total > p.room) {
+    if (lent) {
+      lent = false;
+      plan.cut(limit);
+      if ((rc = ensure_fq(sc, st, at_group + plan.bytes))) return rc;
+      base = static_cast<char *>(sc->fq);
+    }
     if ((rc = ensure_fout(sc, st, *total))) return rc;
     p.room = sc->fcap;
     p.out_pos = sc->fpos;
     p.out_state = sc->fstate;
-    launch_fetch_write(p, st);
-    CK_LAUNCH();
+    if (plan.groups.size() == 1) {  // counted, and nothing written over it
+      launch_fetch_write(p, st);
+      CK_LAUNCH();
+    } else if ((rc = run(true))) {
+      return rc;
+    }
     CK(cudaStreamSynchronize(st));
   }
   return CUBLOX_OK;
@@ -1669,15 +1842,13 @@ int cublox_b200::detail::fetch_into(cublox_grid *g, cudaStream_t st, const float
 }
 
 size_t cublox_b200::detail::fetch_block_bytes(int centres) {
-  // boxes of 32 x 32 columns of up to 32 levels (1.5 m at 0.1 m), overlapping
-  // 5 tiles along x
-  const size_t n = static_cast<size_t>(std::max(centres, 0));
-  return FetchBlock(n, 5 * n, 32 * 32 * n, 32 * 32 * n, 32 * n).bytes;
+  return (static_cast<size_t>(800) << 10) + 208 * static_cast<size_t>(std::max(centres, 0));
 }
 
 int cublox_b200::detail::reserve_fetch(FetchScratch *sc, int centres, int64_t samples,
                                        cudaStream_t st) {
-  int rc = ensure_fq(sc, st, fetch_block_bytes(centres));
+  sc->fq_limit = fetch_block_bytes(centres);
+  int rc = ensure_fq(sc, st, sc->fq_limit);
   if (!rc)
     rc = ensure_pinned(&sc->hoff, &sc->hoff_bytes,
                        sizeof(long long) * (static_cast<size_t>(std::max(centres, 0)) + 1));

@@ -35,7 +35,8 @@ namespace {
 
 // A column: where it is, and what its candidates share.
 struct Column {
-  int rx, ry;       // row and column within the query's box
+  int rx;           // row within the query's box
+  long long at;     // among the query's columns in this launch
   int addr;         // address terms of x and y
   float px, py;     // centre position
   float dx, dy;     // offset from the query's centre
@@ -54,18 +55,26 @@ __device__ __forceinline__ void axis_offset(const FetchParams &p, int g, float c
   d = (p.fp & kFpFetchDFma) ? ffma(t, p.res, -c) : fsub(pos, c);
 }
 
-// This lane's column in tile (tx, ty) of the query's box.
-__device__ __forceinline__ Column column_of(const FetchParams &p, const FetchQuery &q, int tx, int ty,
-                                            int lane) {
+// The first of the columns of row r of unit `unit`'s tile.
+__device__ __forceinline__ long long first_column(const FetchParams &p, const FetchQuery &q, int unit,
+                                                  int r) {
+  return static_cast<long long>(((unit - q.u0) << p.lt[0]) + r) * q.n[1];
+}
+
+// This lane's column in tile (tx, ty) of the query's box, tx unit `unit`'s.
+__device__ __forceinline__ Column column_of(const FetchParams &p, const FetchQuery &q, int unit, int tx,
+                                            int ty, int lane) {
   Column c;
-  const int sx = (tx << p.lt[0]) + (lane >> p.lt[1]);
+  const int r = lane >> p.lt[1];
+  const int sx = (tx << p.lt[0]) + r;
   const int sy = (ty << p.lt[1]) + (lane & ((1 << p.lt[1]) - 1));
   c.valid = (lane >> (p.lt[0] + p.lt[1])) == 0 && sx < p.map[0] && sy < p.map[1];
   const int gx = slot_global(p, 0, sx), gy = slot_global(p, 1, sy);
   c.rx = gx - q.g0[0];
-  c.ry = gy - q.g0[1];
+  const int ry = gy - q.g0[1];
   c.valid = c.valid && static_cast<unsigned>(c.rx) < static_cast<unsigned>(q.n[0]) &&
-            static_cast<unsigned>(c.ry) < static_cast<unsigned>(q.n[1]);
+            static_cast<unsigned>(ry) < static_cast<unsigned>(q.n[1]);
+  c.at = first_column(p, q, unit, r) + ry;
   c.addr = vox_axis(p.lay, 0, sx) + vox_axis(p.lay, 1, sy);
   axis_offset(p, gx, q.c[0], c.px, c.dx);
   axis_offset(p, gy, q.c[1], c.py, c.dy);
@@ -81,7 +90,6 @@ __device__ __forceinline__ Column column_of(const FetchParams &p, const FetchQue
 // kPinned: the sphere test's sum of squares is the pinned fma(z, z, fma(x, x,
 // y * y)).
 constexpr int kBatch = 8;
-constexpr int kFetchCtas = 148 * 8;
 
 struct Levels {
   uint32_t keep, occupied, free_;
@@ -145,17 +153,16 @@ __device__ __forceinline__ int last_tile(const FetchQuery &q) {
   return q.nt[1] * static_cast<int>(blockIdx.y + 1) / static_cast<int>(gridDim.y);
 }
 
-// For each row of tile tx along x: the prefix over its columns, and its
-// total.
-__device__ __forceinline__ void unit_rows(const FetchParams &p, const FetchQuery &q, int tx, int warp,
-                                          int warps, int lane) {
+// For each row of unit `unit`'s tile tx along x: the prefix over its columns,
+// and its total.
+__device__ __forceinline__ void unit_rows(const FetchParams &p, const FetchQuery &q, int unit, int tx,
+                                          int warp, int warps, int lane) {
   for (int r = warp; r < 1 << p.lt[0]; r += warps) {
     const int sx = (tx << p.lt[0]) + r;
     const int rx = slot_global(p, 0, sx) - q.g0[0];
     if (sx >= p.map[0] || static_cast<unsigned>(rx) >= static_cast<unsigned>(q.n[0])) continue;
-    const int sum =
-        warp_prefix(p.col + q.col0 + static_cast<long long>(rx) * q.n[1], q.n[1], lane);
-    if (lane == 0) p.row[q.row0 + rx] = sum;
+    const int sum = warp_prefix(p.col + q.col0 + first_column(p, q, unit, r), q.n[1], lane);
+    if (lane == 0 && !p.rows_done) p.row[q.row0 + rx] = sum;
   }
 }
 
@@ -171,8 +178,7 @@ __global__ void __launch_bounds__(256) fetch_count_kernel(const __grid_constant_
   int *col = p.col + q.col0;
   const int j1 = last_tile(q);
   for (int j = first_tile(q) + warp; j < j1; j += warps) {
-    const Column c = column_of(p, q, tx, ring(q.t0[1] + j, tiles_y), lane);
-    const long long at = static_cast<long long>(c.rx) * q.n[1] + c.ry;
+    const Column c = column_of(p, q, unit.y, tx, ring(q.t0[1] + j, tiles_y), lane);
     const int words = (q.n[2] + 31) >> 5;
     int n = 0;
     for (int k0 = 0; k0 < q.n[2]; k0 += 32) {
@@ -181,13 +187,13 @@ __global__ void __launch_bounds__(256) fetch_count_kernel(const __grid_constant_
         keep |= column_levels<kPinned>(p, q, c, q.g0[2] + k0 + k, ring(s0 + k0 + k, p.map[2]),
                                        q.n[2] - k0 - k).keep << k;
       n += __popc(keep);
-      if (p.mask && c.valid) p.mask[q.mask0 + at * words + (k0 >> 5)] = keep;
+      if (p.mask && c.valid) p.mask[q.mask0 + c.at * words + (k0 >> 5)] = keep;
     }
-    if (c.valid) col[at] = n;
+    if (c.valid) col[c.at] = n;
   }
   if (gridDim.y > 1) return;  // the unit's rows are not done: fetch_columns_kernel
   __syncthreads();            // the CTA's own global writes: its rows' columns
-  unit_rows(p, q, tx, warp, warps, lane);
+  unit_rows(p, q, unit.y, tx, warp, warps, lane);
 }
 
 // The row prefixes of units whose columns several CTAs counted.
@@ -195,7 +201,7 @@ __global__ void __launch_bounds__(256) fetch_columns_kernel(const __grid_constan
   const int2 unit = p.units[blockIdx.x];
   const FetchQuery q = p.queries[unit.x];
   const int tiles_x = (p.map[0] + (1 << p.lt[0]) - 1) >> p.lt[0];
-  unit_rows(p, q, ring(q.t0[0] + unit.y, tiles_x), threadIdx.x >> 5, blockDim.x >> 5,
+  unit_rows(p, q, unit.y, ring(q.t0[0] + unit.y, tiles_x), threadIdx.x >> 5, blockDim.x >> 5,
             threadIdx.x & 31);
 }
 
@@ -211,8 +217,8 @@ __global__ void __launch_bounds__(256) fetch_rows_kernel(const __grid_constant__
   if (i < p.nq) query_rows(p, i, threadIdx.x & 31);
 }
 
-// One CTA: offsets[i] = samples the queries before i keep, offsets[nq] = all.
-// Up to 32 queries' rows are done here too.
+// One CTA: offsets[i] = samples the fetch's queries before i keep, offsets[nq]
+// = those up to here.  Up to 32 queries' rows are done here too.
 __global__ void __launch_bounds__(1024) fetch_offsets_kernel(const __grid_constant__ FetchParams p) {
   __shared__ long long sums[32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -220,7 +226,7 @@ __global__ void __launch_bounds__(1024) fetch_offsets_kernel(const __grid_consta
     if (warp < p.nq) query_rows(p, warp, lane);
     __syncthreads();
   }
-  long long carry = 0;
+  long long carry = p.first ? 0 : p.offsets[0];  // written back below, the same
   for (int i0 = 0; i0 < p.nq; i0 += 1024) {
     const int i = i0 + threadIdx.x;
     const long long x = i < p.nq ? p.kept[i] : 0;
@@ -258,16 +264,15 @@ __global__ void __launch_bounds__(256) fetch_write_kernel(const __grid_constant_
   const long long base = p.offsets[unit.x];
   const int j1 = last_tile(q);
   for (int j = first_tile(q) + warp; j < j1; j += warps) {
-    const Column c = column_of(p, q, tx, ring(q.t0[1] + j, tiles_y), lane);
-    const long long at = static_cast<long long>(c.rx) * q.n[1] + c.ry;
+    const Column c = column_of(p, q, unit.y, tx, ring(q.t0[1] + j, tiles_y), lane);
     const int words = (q.n[2] + 31) >> 5;
     int rank = p.cap;  // of the column's next sample within the query
-    if (c.valid) rank = p.row[q.row0 + c.rx] + p.col[q.col0 + at];
+    if (c.valid) rank = p.row[q.row0 + c.rx] + p.col[q.col0 + c.at];
     for (int k0 = 0; k0 < q.n[2]; k0 += 32) {
       // 32 levels: bit k of keep, occupied and free
       uint32_t keep = 0, occupied = 0, free_ = 0;
       if (p.mask) {  // one state wanted: the count kept the masks
-        if (c.valid) keep = p.mask[q.mask0 + at * words + (k0 >> 5)];
+        if (c.valid) keep = p.mask[q.mask0 + c.at * words + (k0 >> 5)];
         occupied = p.filter == 2 ? keep : 0u;
         free_ = p.filter == 1 ? keep : 0u;
       }
@@ -304,26 +309,28 @@ __global__ void __launch_bounds__(256) fetch_write_kernel(const __grid_constant_
 
 }  // namespace
 
-// CTAs per unit: enough that few units (one large sphere) fill the GPU with
-// kFetchCtas (a 25 m sphere's count: 143 us on its 63 units, 93 on 592 CTAs,
-// 74 on 1,184), at most one per 8 tiles (a CTA's warps).
+// CTAs per unit: enough that few units (one large sphere) fill the GPU with 8
+// an SM (a 25 m sphere's count: 143 us on its 63 units, 93 on 592 CTAs, 74 on
+// 1,184), at most one per 8 tiles (a CTA's warps).
 static int fetch_split(const FetchParams &p) {
-  const int want = (kFetchCtas + p.nu - 1) / p.nu;
+  const int want = (p.ctas + p.nu - 1) / p.nu;
   const int most = (p.most_tiles + 7) / 8;
   return want < most ? want : most;
 }
 
 void launch_fetch_count(const FetchParams &p, cudaStream_t s) {
+  if (p.nu <= 0) return;
+  const dim3 grid(p.nu, fetch_split(p));
+  const int block = 32 * (p.most_tiles < 8 ? p.most_tiles : 8);
+  if (((p.fp >> kFpFetchSosShift) & 7u) == kSosFxFz)
+    fetch_count_kernel<true><<<grid, block, 0, s>>>(p);
+  else
+    fetch_count_kernel<false><<<grid, block, 0, s>>>(p);
+  if (grid.y > 1) fetch_columns_kernel<<<p.nu, 256, 0, s>>>(p);
+}
+
+void launch_fetch_offsets(const FetchParams &p, cudaStream_t s) {
   if (p.nq <= 0) return;
-  if (p.nu > 0) {
-    const dim3 grid(p.nu, fetch_split(p));
-    const int block = 32 * (p.most_tiles < 8 ? p.most_tiles : 8);
-    if (((p.fp >> kFpFetchSosShift) & 7u) == kSosFxFz)
-      fetch_count_kernel<true><<<grid, block, 0, s>>>(p);
-    else
-      fetch_count_kernel<false><<<grid, block, 0, s>>>(p);
-    if (grid.y > 1) fetch_columns_kernel<<<p.nu, 256, 0, s>>>(p);
-  }
   if (p.nq > 32) fetch_rows_kernel<<<(p.nq + 7) / 8, 256, 0, s>>>(p);
   fetch_offsets_kernel<<<1, 1024, 0, s>>>(p);
 }

@@ -12,12 +12,15 @@
 #include "kernels.cuh"
 
 namespace cublox_b200 {
-// Device scratch of a sphere fetch: the query block (queries | work units |
-// columns | rows | samples per query | offsets) and the sample outputs.  A grid grows its own on demand; the server owns one, sized when
-// it is created, shared by its fetches (they run one at a time).
+// Device scratch of a sphere fetch: the query block (samples per query |
+// offsets | queries, work units, rows, columns and level masks of the part of
+// the fetch that is in hand), which is bounded, and the sample outputs.  A grid
+// grows its own on demand; the server owns one, sized when it is created,
+// shared by its fetches (they run one at a time).
 struct FetchScratch {
   void *fq = nullptr;
   size_t fq_bytes = 0;
+  size_t fq_limit = 0;  // the block's bound (0: a grid's own)
   float *fpos = nullptr;
   uint8_t *fstate = nullptr;
   int64_t fcap = 0;
@@ -200,8 +203,8 @@ int attach_voxels(cublox_grid *g, VoxelBuffers *in, const float *occ_host);
 int fetch_into(cublox_grid *g, cudaStream_t st, const float *centers, int nq, float radius,
                int filter, int max_results, std::vector<int64_t> &offsets,
                const std::function<void *(size_t)> &room, FetchScratch *sc = nullptr);
-// Device bytes of the query block of a fetch of that many centres (of up to
-// 1.5 m at 0.1 m; larger boxes grow it).
+// Device bytes of a server's query block for fetches of up to that many
+// centres, of any radius.
 size_t fetch_block_bytes(int centres);
 // Size `sc` for fetches of up to `centres` centres and `samples` samples, so
 // that such fetches allocate nothing.

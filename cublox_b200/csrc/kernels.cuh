@@ -104,13 +104,15 @@ struct ClearParams {
 };
 
 // One sphere of a fetch: its centre, squared radius and candidate box, and
-// the tiles (of 2^lt[0] x 2^lt[1] slots) that the box overlaps.
+// the tiles (of 2^lt[0] x 2^lt[1] slots) that the box overlaps.  A unit of work
+// is a tile along x; its columns, 2^lt[0] rows of n[1], lie together.
 struct FetchQuery {
   float c[3], r2;
   int g0[3], n[3];  // first global index and extent per axis (0: empty)
   int t0[2], nt[2]; // first tile and tiles (around the ring) along x and y
+  int u0;           // the first of the query's units in this launch
   long long row0;   // the query's first row in FetchParams::row
-  long long col0;   // and column in FetchParams::col
+  long long col0;   // unit u0's first column in FetchParams::col
   long long mask0;  // and word in FetchParams::mask
 };
 
@@ -133,8 +135,11 @@ struct FetchParams {
   int *col;           // per column: samples before it in its row
   uint32_t *mask;     // one state wanted: per column, a bit per level kept; else null
   int *row;           // per row: samples before it in its query
+  int rows_done;      // the rows are there already: only the columns are wanted
   int *kept;          // per query: samples it keeps
-  long long *offsets; // per query: where its samples go; [nq]: samples in all
+  long long *offsets; // per query: where its samples go; [nq]: samples up to there
+  int first;          // the queries are the fetch's first (else offsets[0] is known)
+  int ctas;           // CTAs that a launch should have
   long long room;     // samples the outputs hold; more are not written
   float *out_pos;
   uint8_t *out_state;
@@ -201,8 +206,10 @@ int kernel_binary_version();
 void launch_step_count(const RayParams &p, cudaStream_t s);
 void launch_apply(const ApplyParams &p, cudaStream_t s);
 void launch_clear(const ClearParams &p, cudaStream_t s);
-// Sphere fetch (fetch.cu): where each sample goes, then the samples.
+// Sphere fetch (fetch.cu): samples per column and row, where each query's
+// samples go, then the samples.
 void launch_fetch_count(const FetchParams &p, cudaStream_t s);
+void launch_fetch_offsets(const FetchParams &p, cudaStream_t s);
 void launch_fetch_write(const FetchParams &p, cudaStream_t s);
 void launch_query(const QueryParams &p, cudaStream_t s);
 // Sensor-frame cloud -> world-frame SoA (the reference driver's

@@ -208,7 +208,10 @@ int cublox_grid_fetch_viz(cublox_grid *g, const float center[3], float radius, i
  * fetchOccupancyAround once per centre).  out_offsets gets n_centers+1
  * entries; query q's samples are [out_offsets[q], out_offsets[q+1]).
  * Output buffers are host pointers.  If capacity is too small the call
- * fills out_offsets and returns CUBLOX_ERR_INVALID without samples.       */
+ * fills out_offsets and returns CUBLOX_ERR_INVALID without samples.  Besides
+ * 13 B a sample, a grid keeps up to 64 MiB of device scratch for its fetches
+ * and 12 B per centre; what does not fit at once is fetched in several
+ * launches, and where that much cannot be allocated, in 1 MiB.             */
 int cublox_grid_fetch_batch(cublox_grid *g, const float *centers,
                             int n_centers, float radius, int filter,
                             int max_results, int64_t *out_offsets,
@@ -395,8 +398,8 @@ int cublox_batch_stream(const cublox_batch *b, void **stream);
  * max_tick_points) in one batched launch sequence, the next tick being
  * queued while the previous one still runs.  Maps are admitted to device
  * memory against hbm_budget_bytes (12 B a voxel, the tick's point buffers
- * and the fetch buffers maps keep between requests; a fetch in flight may
- * exceed it by its own output buffers until it ends): when a map's
+ * and the scratch that all fetches share, which only a fetch of more centres
+ * or samples than configured exceeds): when a map's
  * buffers do not fit, least recently used idle maps are evicted to host
  * memory and restored bit for bit when next used.  Per map, requests take
  * effect in submission order, and every result equals that of the same
