@@ -1562,10 +1562,12 @@ static int ensure_pinned(void **p, size_t *have, size_t bytes) {
 }
 
 // Finds the fetch's samples: sc->hoff[0 .. nq] are the queries' offsets, *total
-// the last of them, and, with `write`, the samples are in sc->fpos and
-// sc->fstate when it returns.  What an earlier fetch_begin left there is gone.
+// the last of them, and, with `write` and unless there are more than `most`,
+// the samples are in sc->fpos and sc->fstate when it returns.  What an earlier
+// fetch_begin left there is gone.
 static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int nq, float radius,
-                     int filter, int max_results, bool write, FetchScratch *sc, int64_t *total) {
+                     int filter, int max_results, bool write, FetchScratch *sc, int64_t *total,
+                     int64_t most = std::numeric_limits<int64_t>::max()) {
   *total = 0;
   if (!g || (nq > 0 && !centers)) return fail(CUBLOX_ERR_INVALID, "fetch: null argument");
   if (!sc) sc = &g->fs;
@@ -1711,7 +1713,7 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
                      cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   *total = off[nq];
-  if (write && *total > p.room) {
+  if (write && *total > p.room && *total <= most) {
     if (lent) {
       lent = false;
       plan.cut(limit);
@@ -1934,7 +1936,8 @@ int cublox_grid_fetch(cublox_grid *g, const float center[3], float radius,
   if (n_out) *n_out = 0;
   if (!g || !center) return fail(CUBLOX_ERR_INVALID, "cublox_grid_fetch: null argument");
   int64_t kept = 0;
-  int rc = fetch_run(g, g->stream, center, 1, radius, filter, max_results, true, &g->fs, &kept);
+  int rc = fetch_run(g, g->stream, center, 1, radius, filter, max_results, true, &g->fs, &kept,
+                     capacity);
   if (rc) return rc;
   if (kept > capacity)
     return fail(CUBLOX_ERR_INVALID, "cublox_grid_fetch: capacity " + std::to_string(capacity) +
@@ -1946,9 +1949,9 @@ int cublox_grid_fetch(cublox_grid *g, const float center[3], float radius,
 
 // A fetch of many centres on the grid's own scratch, with its offsets copied out.
 static int fetch_many(cublox_grid *g, const float *centers, int n_centers, float radius, int filter,
-                      int max_results, int64_t *out_offsets, int64_t *total) {
+                      int max_results, int64_t *out_offsets, int64_t *total, int64_t most) {
   const int rc = fetch_run(g, g ? g->stream : nullptr, centers, n_centers, radius, filter,
-                           max_results, true, nullptr, total);
+                           max_results, true, nullptr, total, most);
   if (rc) return rc;
   const long long *off = static_cast<const long long *>(g->fs.hoff);
   std::copy(off, off + std::max(n_centers, 0) + 1, out_offsets);
@@ -1959,8 +1962,8 @@ int cublox_grid_fetch_begin(cublox_grid *g, const float *centers, int n_centers,
                             int filter, int max_results, int64_t *out_offsets) {
   if (!out_offsets) return fail(CUBLOX_ERR_INVALID, "fetch_begin: null offsets");
   int64_t total = 0;
-  const int rc =
-      fetch_many(g, centers, n_centers, radius, filter, max_results, out_offsets, &total);
+  const int rc = fetch_many(g, centers, n_centers, radius, filter, max_results, out_offsets, &total,
+                            std::numeric_limits<int64_t>::max());
   if (!rc) g->fs.pending = total;
   return rc;
 }
@@ -1979,8 +1982,8 @@ int cublox_grid_fetch_batch(cublox_grid *g, const float *centers,
                             int64_t capacity) {
   if (!out_offsets) return fail(CUBLOX_ERR_INVALID, "fetch_batch: null offsets");
   int64_t total = 0;
-  const int rc =
-      fetch_many(g, centers, n_centers, radius, filter, max_results, out_offsets, &total);
+  const int rc = fetch_many(g, centers, n_centers, radius, filter, max_results, out_offsets, &total,
+                            capacity);
   if (rc) return rc;
   if (total > capacity)
     return fail(CUBLOX_ERR_INVALID, "fetch: output capacity " + std::to_string(capacity) + " < " +
