@@ -1450,12 +1450,9 @@ struct FetchPlan {
   std::vector<FetchGroup> groups;
   std::deque<FetchQuery> parts;  // descriptors of queries in parts
   size_t bytes = 0;              // the largest group's
-  const int row_bits;
   const bool masks;
 
-  FetchPlan(size_t n, int row_bits_, bool masks_) : row_bits(row_bits_), masks(masks_) {
-    queries.reserve(n);
-  }
+  FetchPlan(size_t n, bool masks_) : masks(masks_) { queries.reserve(n); }
 
   // One more query, into the one group that all of them would make.
   void push(FetchQuery &q) {
@@ -1493,7 +1490,7 @@ struct FetchPlan {
       size_t step = nu;
       if (s.bytes() > limit) {  // the same places in each part
         const size_t fixed = with(FetchSizes{}, q, 0, false).bytes() + 512;  // and two roundings
-        const size_t per = sizeof(int2) + sizeof(int) * (static_cast<size_t>(q.n[1]) << row_bits);
+        const size_t per = sizeof(int2) + sizeof(int) * (static_cast<size_t>(q.n[1]) << kFetchTileX);
         step = std::max<size_t>(1, std::min(limit > fixed ? (limit - fixed) / per : 0, nu));
         s = with(FetchSizes{}, q, step, false);
       }
@@ -1514,7 +1511,7 @@ struct FetchPlan {
 
   // The sizes of a group with n_units units of q added.
   FetchSizes with(FetchSizes s, const FetchQuery &q, size_t n_units, bool masked) const {
-    const size_t columns = n_units * (static_cast<size_t>(q.n[1]) << row_bits);
+    const size_t columns = n_units * (static_cast<size_t>(q.n[1]) << kFetchTileX);
     ++s.queries;
     s.units += n_units;
     s.rows += static_cast<size_t>(q.n[0]);
@@ -1580,14 +1577,10 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
   off[0] = 0;
   if (nq == 0) return CUBLOX_OK;
   FetchParams p{};
-  // tiles: the bricks' columns (at most 32, as in every layout of 32-voxel
-  // bricks); in the reference's order, 8 x 4 columns
-  p.lt[0] = g->lay_code == 0 ? 3 : g->lay.lb[0];
-  p.lt[1] = g->lay_code == 0 ? 2 : g->lay.lb[1];
   int low_slot[2];  // of the window's first voxel; a box lies in the window
   for (int a = 0; a < 2; ++a)
     low_slot[a] = global_to_local(g->origin_i[a] - g->half[a], g->map[a], g->half[a]) + g->half[a];
-  FetchPlan plan(static_cast<size_t>(nq), p.lt[0], write && filter >= 0);
+  FetchPlan plan(static_cast<size_t>(nq), write && filter >= 0);
   for (int i = 0; i < nq; ++i) {
     const float *c = centers + 3 * static_cast<size_t>(i);
     const QueryBox b = plan_query(g, c, radius);
@@ -1604,14 +1597,15 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
       continue;
     }
     for (int a = 0; a < 2; ++a) {
-      const int m = g->map[a], tiles = (m + (1 << p.lt[a]) - 1) >> p.lt[a];
+      const int m = g->map[a], log2 = a == 0 ? kFetchTileX : kFetchTileY;
+      const int tiles = (m + (1 << log2) - 1) >> log2;
       int first = low_slot[a] + (q.g0[a] - (g->origin_i[a] - g->half[a]));
       if (first >= m) first -= m;
       int last = first + q.n[a] - 1;
       if (last >= m) last -= m;
-      q.t0[a] = first >> p.lt[a];
+      q.t0[a] = first >> log2;
       // around the ring where the box wraps; its two ends may share a tile
-      const int span = (last >> p.lt[a]) - q.t0[a] + 1 + (last < first ? tiles : 0);
+      const int span = (last >> log2) - q.t0[a] + 1 + (last < first ? tiles : 0);
       q.nt[a] = std::min(span, tiles);
     }
     plan.push(q);

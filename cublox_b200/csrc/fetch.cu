@@ -3,8 +3,8 @@
 // (x, y, z) order.
 //
 // A lane takes one (x, y) column of the box and walks it upwards; a warp's
-// lanes are the columns of one tile of the voxel layout's bricks (8 x 4 by
-// default), so that a level of the tile is one 128-byte line.  What is the
+// lanes are the columns of a tile of 8 x 4 slots, so that a level of the tile is
+// one 128-byte line of the default voxel layout's bricks.  What is the
 // same for a column (its squared offset, its address terms) is computed once
 // per column, and nothing is divided per candidate.  The launches:
 //   count    samples per column, then a prefix over the columns of each x row
@@ -56,25 +56,24 @@ __device__ __forceinline__ void axis_offset(const FetchParams &p, int g, float c
 }
 
 // The first of the columns of row r of unit `unit`'s tile.
-__device__ __forceinline__ long long first_column(const FetchParams &p, const FetchQuery &q, int unit,
-                                                  int r) {
-  return static_cast<long long>(((unit - q.u0) << p.lt[0]) + r) * q.n[1];
+__device__ __forceinline__ long long first_column(const FetchQuery &q, int unit, int r) {
+  return static_cast<long long>(((unit - q.u0) << kFetchTileX) + r) * q.n[1];
 }
 
 // This lane's column in tile (tx, ty) of the query's box, tx unit `unit`'s.
 __device__ __forceinline__ Column column_of(const FetchParams &p, const FetchQuery &q, int unit, int tx,
                                             int ty, int lane) {
   Column c;
-  const int r = lane >> p.lt[1];
-  const int sx = (tx << p.lt[0]) + r;
-  const int sy = (ty << p.lt[1]) + (lane & ((1 << p.lt[1]) - 1));
-  c.valid = (lane >> (p.lt[0] + p.lt[1])) == 0 && sx < p.map[0] && sy < p.map[1];
+  const int r = lane >> kFetchTileY;
+  const int sx = (tx << kFetchTileX) + r;
+  const int sy = (ty << kFetchTileY) + (lane & ((1 << kFetchTileY) - 1));
+  c.valid = sx < p.map[0] && sy < p.map[1];
   const int gx = slot_global(p, 0, sx), gy = slot_global(p, 1, sy);
   c.rx = gx - q.g0[0];
   const int ry = gy - q.g0[1];
   c.valid = c.valid && static_cast<unsigned>(c.rx) < static_cast<unsigned>(q.n[0]) &&
             static_cast<unsigned>(ry) < static_cast<unsigned>(q.n[1]);
-  c.at = first_column(p, q, unit, r) + ry;
+  c.at = first_column(q, unit, r) + ry;
   c.addr = vox_axis(p.lay, 0, sx) + vox_axis(p.lay, 1, sy);
   axis_offset(p, gx, q.c[0], c.px, c.dx);
   axis_offset(p, gy, q.c[1], c.py, c.dy);
@@ -157,11 +156,11 @@ __device__ __forceinline__ int last_tile(const FetchQuery &q) {
 // and its total.
 __device__ __forceinline__ void unit_rows(const FetchParams &p, const FetchQuery &q, int unit, int tx,
                                           int warp, int warps, int lane) {
-  for (int r = warp; r < 1 << p.lt[0]; r += warps) {
-    const int sx = (tx << p.lt[0]) + r;
+  for (int r = warp; r < 1 << kFetchTileX; r += warps) {
+    const int sx = (tx << kFetchTileX) + r;
     const int rx = slot_global(p, 0, sx) - q.g0[0];
     if (sx >= p.map[0] || static_cast<unsigned>(rx) >= static_cast<unsigned>(q.n[0])) continue;
-    const int sum = warp_prefix(p.col + q.col0 + first_column(p, q, unit, r), q.n[1], lane);
+    const int sum = warp_prefix(p.col + q.col0 + first_column(q, unit, r), q.n[1], lane);
     if (lane == 0 && !p.rows_done) p.row[q.row0 + rx] = sum;
   }
 }
@@ -171,8 +170,8 @@ __global__ void __launch_bounds__(256) fetch_count_kernel(const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int2 unit = p.units[blockIdx.x];
   const FetchQuery q = p.queries[unit.x];
-  const int tiles_x = (p.map[0] + (1 << p.lt[0]) - 1) >> p.lt[0];
-  const int tiles_y = (p.map[1] + (1 << p.lt[1]) - 1) >> p.lt[1];
+  const int tiles_x = (p.map[0] + (1 << kFetchTileX) - 1) >> kFetchTileX;
+  const int tiles_y = (p.map[1] + (1 << kFetchTileY) - 1) >> kFetchTileY;
   const int tx = ring(q.t0[0] + unit.y, tiles_x);
   const int s0 = global_to_local(q.g0[2], p.map[2], p.half[2]) + p.half[2];
   int *col = p.col + q.col0;
@@ -200,7 +199,7 @@ __global__ void __launch_bounds__(256) fetch_count_kernel(const __grid_constant_
 __global__ void __launch_bounds__(256) fetch_columns_kernel(const __grid_constant__ FetchParams p) {
   const int2 unit = p.units[blockIdx.x];
   const FetchQuery q = p.queries[unit.x];
-  const int tiles_x = (p.map[0] + (1 << p.lt[0]) - 1) >> p.lt[0];
+  const int tiles_x = (p.map[0] + (1 << kFetchTileX) - 1) >> kFetchTileX;
   unit_rows(p, q, unit.y, ring(q.t0[0] + unit.y, tiles_x), threadIdx.x >> 5, blockDim.x >> 5,
             threadIdx.x & 31);
 }
@@ -257,8 +256,8 @@ __global__ void __launch_bounds__(256) fetch_write_kernel(const __grid_constant_
   const uint32_t lt = (1u << lane) - 1u;  // lanes below this one
   const int2 unit = p.units[blockIdx.x];
   const FetchQuery q = p.queries[unit.x];
-  const int tiles_x = (p.map[0] + (1 << p.lt[0]) - 1) >> p.lt[0];
-  const int tiles_y = (p.map[1] + (1 << p.lt[1]) - 1) >> p.lt[1];
+  const int tiles_x = (p.map[0] + (1 << kFetchTileX) - 1) >> kFetchTileX;
+  const int tiles_y = (p.map[1] + (1 << kFetchTileY) - 1) >> kFetchTileY;
   const int tx = ring(q.t0[0] + unit.y, tiles_x);
   const int s0 = global_to_local(q.g0[2], p.map[2], p.half[2]) + p.half[2];
   const long long base = p.offsets[unit.x];

@@ -103,9 +103,16 @@ struct ClearParams {
   int nbr[3];        // bricks per axis
 };
 
+// Slots of a fetch's tiles along x and y, log2: 32 columns, a line of the
+// default layout's bricks.  In other layouts tiles of their bricks' columns
+// gain nothing, and are half empty where bricks are more than a voxel high
+// (2 x 2 x 8 bricks: the count of a 25 m sphere and its round trip 562 us,
+// 120 with these tiles, 121 in the default layout).
+constexpr int kFetchTileX = 3, kFetchTileY = 2;
+
 // One sphere of a fetch: its centre, squared radius and candidate box, and
-// the tiles (of 2^lt[0] x 2^lt[1] slots) that the box overlaps.  A unit of work
-// is a tile along x; its columns, 2^lt[0] rows of n[1], lie together.
+// the tiles that the box overlaps.  A unit of work is a tile along x; its
+// columns, a tile's rows of n[1], lie together.
 struct FetchQuery {
   float c[3], r2;
   int g0[3], n[3];  // first global index and extent per axis (0: empty)
@@ -123,7 +130,6 @@ struct FetchParams {
   const int2 *units;  // a query and a tile along x, within the query's
   int nu;
   int most_tiles;     // along y, of any query
-  int lt[2];          // log2 of a tile's sides (columns), at most 32 columns
   int win[3], half[3], map[3];
   float res;
   int ctr;
