@@ -27,6 +27,8 @@
 #include <cstdint>
 #include <cstring>
 #include <deque>
+#include <iterator>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -110,6 +112,23 @@ struct Tick {
 
 }  // namespace
 
+// Pinned host memory allocated with `device` current (the calling thread's own
+// current device is put back afterwards).
+static cudaError_t alloc_pinned(size_t bytes, int device, char **out) {
+  int prev = -1;
+  if (cudaGetDevice(&prev) != cudaSuccess) {
+    cudaGetLastError();
+    prev = -1;
+  }
+  const bool switched = prev >= 0 && prev != device && cudaSetDevice(device) == cudaSuccess;
+  void *p = nullptr;
+  const cudaError_t e = bytes ? cublox_b200::detail::hmalloc(&p, bytes) : cudaSuccess;
+  if (switched) cudaSetDevice(prev);
+  if (e != cudaSuccess) cudaGetLastError();
+  *out = static_cast<char *>(p);
+  return e;
+}
+
 // Pinned host blocks for scan points, reused by size class (64 KiB << c).
 // A scan submitted into one is copied to the device by DMA straight from
 // it, so the worker thread copies nothing for a one-scan tick.  Blocks are
@@ -125,23 +144,9 @@ struct PinnedPool {
   char *arena = nullptr;
   size_t arena_bytes = 0, carved = 0;
 
-  // Allocates the arena with `device` current (the calling thread's own
-  // current device is put back afterwards).
   int init(size_t bytes, int device) {
-    int prev = -1;
-    if (cudaGetDevice(&prev) != cudaSuccess) {
-      cudaGetLastError();
-      prev = -1;
-    }
-    const bool switched = prev >= 0 && prev != device && cudaSetDevice(device) == cudaSuccess;
-    void *p = nullptr;
-    const cudaError_t e = bytes ? cublox_b200::detail::hmalloc(&p, bytes) : cudaSuccess;
-    if (switched) cudaSetDevice(prev);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
+    if (alloc_pinned(bytes, device, &arena) != cudaSuccess)
       return fail(CUBLOX_ERR_NOMEM, "server: pinned arena allocation failed");
-    }
-    arena = static_cast<char *>(p);
     arena_bytes = bytes;
     return CUBLOX_OK;
   }
@@ -175,9 +180,63 @@ struct PinnedPool {
   }
 };
 
+// Pinned host memory for the results of fetches, apart from the scans': a
+// result is held until its request is released.  Pieces of any size, first
+// fit, and neighbours that are given back become one piece again.  A result
+// that finds no room is kept in pageable memory.
+struct ResultArena {
+  static constexpr size_t kMost = size_t(32) << 20, kGrain = size_t(4) << 10;
+  std::mutex mu;
+  char *base = nullptr;
+  std::map<size_t, size_t> free;  // start, bytes
+
+  // Without the memory, every result is pageable.
+  void init(size_t bytes, int device) {
+    bytes &= ~(kGrain - 1);
+    if (bytes && alloc_pinned(bytes, device, &base) == cudaSuccess) free[0] = bytes;
+  }
+  static size_t grains(size_t bytes) { return (bytes + kGrain - 1) & ~(kGrain - 1); }
+  bool take(size_t bytes, size_t *at) {
+    bytes = grains(bytes);
+    std::lock_guard<std::mutex> lk(mu);
+    for (auto it = free.begin(); it != free.end(); ++it) {
+      if (it->second < bytes) continue;
+      *at = it->first;
+      const size_t left = it->second - bytes;
+      free.erase(it);
+      if (left) free[*at + bytes] = left;
+      return true;
+    }
+    return false;
+  }
+  void give(size_t at, size_t bytes) {
+    bytes = grains(bytes);
+    std::lock_guard<std::mutex> lk(mu);
+    auto next = free.lower_bound(at);
+    if (next != free.end() && at + bytes == next->first) {
+      bytes += next->second;
+      next = free.erase(next);
+    }
+    if (next != free.begin()) {
+      auto before = std::prev(next);
+      if (before->first + before->second == at) {
+        before->second += bytes;
+        return;
+      }
+    }
+    free[at] = bytes;
+  }
+  void release_all() {
+    cublox_b200::detail::hfree(base);
+    base = nullptr;
+    free.clear();
+  }
+};
+
 struct cublox_server {
   cublox_server_config cfg{};
-  PinnedPool pinned;  // scan points
+  PinnedPool pinned;    // scan points
+  ResultArena results;  // fetch results (before reqs, which give theirs back)
   cublox_b200::FetchScratch fscratch;  // shared by fetches (one at a time)
   int reserved_maps = 0;  // maps the batch's item buffers are sized for
   cublox_batch *batch = nullptr;
@@ -422,14 +481,14 @@ void defer(cublox_server *s, Request *r) {
   s->maps[r->map]->queue.push_front(r);
 }
 
-// Host memory for a fetch's result: a block of the pinned pool, which the
-// device copies into directly and which goes back when the request is
-// released, or, where the pool has none, pageable memory.
+// Host memory for a fetch's result: a piece of the results' pinned arena, which
+// the device copies into directly and which goes back when the request is
+// released, or, where the arena has none, pageable memory.
 void *result_room(cublox_server *s, Request *r, size_t bytes) {
-  int cls = -1;
-  if (float *p = s->pinned.take(bytes, &cls))
-    r->fresult = std::shared_ptr<char>(reinterpret_cast<char *>(p), [s, p, cls](char *) {
-      s->pinned.give(p, cls);
+  size_t at = 0;
+  if (s->results.take(bytes, &at))
+    r->fresult = std::shared_ptr<char>(s->results.base + at, [s, at, bytes](char *) {
+      s->results.give(at, bytes);
     });
   else
     r->fresult = std::shared_ptr<char>(new (std::nothrow) char[bytes], std::default_delete<char[]>());
@@ -728,6 +787,8 @@ int cublox_server_create(const cublox_server_config *cfg, cublox_server **out) {
   if (!rc)
     rc = cublox_b200::detail::reserve_fetch(&s->fscratch, s->cfg.max_fetch_centres,
                                             s->cfg.max_fetch_samples, s->fstream);
+  if (!rc)
+    s->results.init(std::min<size_t>(ResultArena::kMost, s->cfg.pinned_pool_bytes / 8), s->device);
   if (rc) {
     const std::string msg = cublox_last_error();
     cublox_b200::detail::free_fetch(&s->fscratch);
@@ -778,6 +839,7 @@ int cublox_server_destroy(cublox_server *s) {
   cublox_batch_destroy(s->batch);
   cublox_b200::detail::free_fetch(&s->fscratch);
   s->pinned.release_all();
+  s->results.release_all();
   cudaStreamDestroy(s->stream);
   cudaStreamDestroy(s->fstream);
   delete s;
