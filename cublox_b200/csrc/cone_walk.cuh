@@ -66,7 +66,10 @@ __device__ __forceinline__ void cone_table(const RayParams &p, int *table) {
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const int m = p.map[a], up = cone_axis_base(p, a, 0), down = cone_axis_base(p, a, 1);
-    const int s0 = global_to_local(p.win[a] - p.half[a], m, p.half[a]) + p.half[a];
+    // slot of the window's far side: the middle's less half, around the ring
+    // (win - half itself may be out of range)
+    const int l0 = global_to_local(p.win[a], m, p.half[a]);
+    const int s0 = l0 < 0 ? l0 + m : l0;
     for (int r = threadIdx.x; r < m + kBlock; r += blockDim.x) {
       if (r >= m) {
         table[up + r] = table[down + r] = 0;
@@ -284,6 +287,15 @@ __device__ __forceinline__ void cone_walk(const RayParams &p, const int *table, 
   RayWalk w;
   if (live && ray_begin(p, ex, ey, ez, w)) {
     ++rays;
+    // Where the sensor's index is 2^31 voxels or more from the window's (one of
+    // them out of range), rel has wrapped around: it does not say where in the
+    // table the voxel's slot is.
+    bool apart = false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const long long d = static_cast<long long>(w.id[a]) - p.win[a];
+      apart = apart || d > INT32_MAX || d < -INT32_MAX;
+    }
     r.he = end_hash(w, p);
     hit = r.he >= 0 && !w.clipped;
     // up to the window, if the sensor is outside it
@@ -303,7 +315,7 @@ __device__ __forceinline__ void cone_walk(const RayParams &p, const int *table, 
     // leave no time finite (below kConeMaxRes the time of a ray's longest axis
     // grows by less than 2e25 a step, in up to 2^33 steps).
     const float inf = inf_f();
-    if (!(p.res < kConeMaxRes) || !(w.tM[0] > -inf) || !(w.tM[1] > -inf) || !(w.tM[2] > -inf) ||
+    if (apart || !(p.res < kConeMaxRes) || !(w.tM[0] > -inf) || !(w.tM[1] > -inf) || !(w.tM[2] > -inf) ||
         !(fminf(w.tM[0], fminf(w.tM[1], w.tM[2])) < inf)) {
       int last = -1;
       while (k < w.max_steps && !at_end(w) && !left_for_good(w, p)) {

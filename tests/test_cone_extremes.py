@@ -48,3 +48,49 @@ def test_times_that_run_out_of_range(n, res, max_range):
     move on.  From 1e25 m on, maps are walked step by step."""
     s = [-2.83568231e18, 1.00390983e9, 0.0]
     _same((3, 3, 3), res, max_range, s, [[0.0, -0.0, 0.0]] * n)
+
+
+LOW, TOP = -2**31, 2**31 - 1
+
+
+@pytest.mark.parametrize("ctr", [False, True])
+@pytest.mark.parametrize("win,sensor", [
+    ((0, 0, 0), (-3e8, 0, 0)), ((0, 0, 0), (0, -3e8, 0)), ((LOW, 0, 0), (-3e8, 0, 0)), ((LOW, 0, 0), (3e8, 0, 0)),
+    ((LOW, LOW, LOW), (-2.1474836e8, -2.1474836e8, -2.1474836e8)), ((TOP, 5, 0), (-3e8, 0, 0)), ((TOP, 5, 0), (3e8, 0, 0)),
+    ((TOP, 0, 0), (2.1474836e8, 0.05, 0.05)), ((LOW + 3, 0, TOP - 2), (-2.1474835e8, 0.05, 2.1474835e8))], ids=str)
+def test_indices_at_the_ends_of_their_range(win, sensor, ctr):
+    """Sensors and windows 2^31 voxels from the origin and from one another: an
+    index saturates, and its distance from the window wraps around.  As the
+    walk of one thread a ray has it, which follows each axis's slot.  No ray
+    reaches the last window."""
+    half, rng = (20, 15, 6), np.random.default_rng(1)
+    s = np.float32(sensor)
+    d = rng.normal(size=(200, 3)) * 200
+    d[:50] *= [1, 1e-3, 1e-3]
+    d[50:100] *= [1e-3, 1, 1e-3]
+    p = (s + d).astype(np.float32)
+    ref, g, b = C.OccupancyGrid(half, 0.1, ctr, None), C.OccupancyGrid(half, 0.1, ctr, None), C.Batch()
+    ref.set_option(C.OPT_RAYCAST, 0)
+    b.set_option(C.BATCH_OPT_SHAPE, 0)
+    bg = b.add_grid(half, 0.1, ctr, None)
+    for x in (ref, g, bg):
+        x.setLogOddsParams(*LO)
+        x.setMaxRaycastRange(1e9)
+        x.set_origin_index(win)
+    ref.update(p, s)
+    g.update(p, s)
+    b.update([bg], [p], [s])
+    want = ref.export().view(np.uint32)
+    assert np.count_nonzero(want) or win == (LOW + 3, 0, TOP - 2)
+    for x in (g, bg):
+        assert np.array_equal(x.export().view(np.uint32), want)
+    if win == (0, 0, 0):  # no index wraps around on the way
+        o = O.OracleGrid(half, 0.1, ctr, None)
+        o.set_log_odds(*LO)
+        o.set_max_range(1e9)
+        o.set_origin_index(win)
+        o.update(p, s)
+        assert np.array_equal(want, o.occ().view(np.uint32))
+    for x in (ref, g):
+        x.close()
+    b.close()
