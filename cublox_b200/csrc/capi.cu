@@ -14,6 +14,7 @@
 #include <deque>
 #include <limits>
 #include <functional>
+#include <mutex>
 #include <string>
 #include <system_error>
 #include <thread>
@@ -1628,7 +1629,15 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
     lent = plan.bytes <= upper;
     if (!lent) plan.cut(limit);
   }
-  rc = ensure_fq(sc, st, at_group + (lent ? 0 : plan.bytes));
+  // A grid's first block also holds one box of the whole map (up to 8 MiB): to
+  // allocate it takes no longer, to replace it by a larger one 0.6 ms.
+  size_t whole = 0;
+  if (!sc->fq && !sc->fq_limit) {
+    whole = sizeof(int) * static_cast<size_t>(g->map[0]) * static_cast<size_t>(g->map[1]) *
+            (1 + (static_cast<size_t>(g->map[2]) + 31) / 32);
+    whole = std::min(whole, static_cast<size_t>(8) << 20);
+  }
+  rc = ensure_fq(sc, st, at_group + std::max(whole, lent ? 0 : plan.bytes));
   if (rc == CUBLOX_ERR_NOMEM && bound > kFetchLeast) {
     plan.cut(least);
     rc = ensure_fq(sc, st, at_group + plan.bytes);
@@ -1729,14 +1738,61 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
   return CUBLOX_OK;
 }
 
-// Device to pageable host memory.  From kThreadedCopy on, through the
-// scratch's pinned buffer in pieces that several threads take in turn, each
-// waiting for its piece's DMA and then copying it out, so that the copies
-// (and the first touch of the caller's fresh pages, which costs more than
-// they do) run side by side and beside the DMA: 54 MB into new arrays 3.4 ms,
-// against 10.9 ms by the runtime's own staging; 1.6 MB takes that 0.14 ms,
-// threads 0.12 to 0.28.
-static int copy_out(cublox_grid *g, cudaStream_t st, FetchScratch *sc,
+// Pinned staging buffers for copy_out, shared by all grids: pinning 4 MB takes
+// 2 to 4 ms, more than most fetches.  Each is used by one copy at a time; up to
+// kIdle wait for the next one (several threads may copy at once).
+class StagingPool {
+ public:
+  // A buffer (all have the same size), or null where there is no memory.
+  void *take(size_t bytes) {
+    for (;;) {
+      void *p = nullptr;
+      {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (idle_.empty()) break;
+        p = idle_.back();
+        idle_.pop_back();
+      }
+      if (mem_kind(p) == 1) return p;  // else a device reset has freed it
+    }
+    void *p = nullptr;
+    if (cublox_b200::detail::hmalloc(&p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    return p;
+  }
+  void give(void *p) {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      if (idle_.size() < kIdle) {
+        idle_.push_back(p);
+        return;
+      }
+    }
+    cublox_b200::detail::hfree(p);
+  }
+
+ private:
+  static constexpr size_t kIdle = 2;
+  std::mutex mu_;
+  std::vector<void *> idle_;
+};
+
+static StagingPool &staging_pool() {
+  static StagingPool *pool = new StagingPool;  // not destroyed: the runtime may be gone by then
+  return *pool;
+}
+
+// Device to pageable host memory.  From kThreadedCopy on, through a pinned
+// buffer in pieces that several threads take in turn, each waiting for its
+// piece's DMA and then copying it out, so that the copies (and the first touch
+// of the caller's fresh pages, which costs more than they do) run side by side
+// and beside the DMA.  To fresh pages / pages in use, ms, and by the runtime's
+// own staging: 6 MB 1.2 / 0.49 (3.0 / 0.43), 12 MB 2.2 / 0.7 (5.9 / 0.82), 54 MB
+// 8.0 / 2.5 (27 / 3.2); 2 MB takes that 1.0 / 0.19, and starting the threads
+// 0.1 to 0.2.
+static int copy_out(cublox_grid *g, cudaStream_t st,
                     const std::pair<const void *, void *> *parts, const size_t *bytes, int n_parts) {
   constexpr size_t kThreadedCopy = static_cast<size_t>(4) << 20;
   constexpr size_t kPiece = static_cast<size_t>(512) << 10;
@@ -1744,7 +1800,11 @@ static int copy_out(cublox_grid *g, cudaStream_t st, FetchScratch *sc,
   size_t all = 0;
   for (int i = 0; i < n_parts; ++i)
     if (parts[i].second) all += bytes[i];
-  if (all < kThreadedCopy) {
+  const int cores = static_cast<int>(std::thread::hardware_concurrency());
+  const int threads = std::max(1, std::min(kMostThreads, cores / 2));
+  char *stage =
+      all < kThreadedCopy ? nullptr : static_cast<char *>(staging_pool().take(kPiece * threads));
+  if (!stage) {
     for (int i = 0; i < n_parts; ++i)
       if (parts[i].second)
         CK(cudaMemcpyAsync(parts[i].second, parts[i].first, bytes[i], cudaMemcpyDeviceToHost, st));
@@ -1761,17 +1821,13 @@ static int copy_out(cublox_grid *g, cudaStream_t st, FetchScratch *sc,
     for (size_t o = 0; parts[i].second && o < bytes[i]; o += kPiece)
       pieces.push_back({static_cast<const char *>(parts[i].first) + o,
                         static_cast<char *>(parts[i].second) + o, std::min(kPiece, bytes[i] - o)});
-  int rc;
-  const int cores = static_cast<int>(std::thread::hardware_concurrency());
-  const int threads = std::max(1, std::min(kMostThreads, cores / 2));
-  if ((rc = ensure_pinned(&sc->hcopy, &sc->hcopy_bytes, kPiece * threads))) return rc;
   std::atomic<size_t> next{0};
   std::atomic<int> error{cudaSuccess};
   auto work = [&](int t) {
     cudaEvent_t ev = nullptr;
     cudaError_t e = cudaSetDevice(g->device);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-    char *h = static_cast<char *>(sc->hcopy) + kPiece * t;
+    char *h = stage + kPiece * t;
     for (size_t i; e == cudaSuccess && (i = next.fetch_add(1)) < pieces.size();) {
       const Piece &p = pieces[i];
       if ((e = cudaMemcpyAsync(h, p.src, p.bytes, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
@@ -1792,13 +1848,15 @@ static int copy_out(cublox_grid *g, cudaStream_t st, FetchScratch *sc,
   }
   work(0);
   for (std::thread &h : helpers) h.join();
+  if (error != cudaSuccess) cudaStreamSynchronize(st);  // copies into the buffer that nobody waited for
   if (prev >= 0 && prev != g->device) cudaSetDevice(prev);
+  staging_pool().give(stage);
   CK(static_cast<cudaError_t>(error.load()));
   return CUBLOX_OK;
 }
 
 // The n samples that fetch_run wrote to host memory (null: not wanted).
-static int fetch_copy(cublox_grid *g, cudaStream_t st, FetchScratch *sc, int64_t samples,
+static int fetch_copy(cublox_grid *g, cudaStream_t st, const FetchScratch *sc, int64_t samples,
                       float *out_pos, uint8_t *out_state) {
   const size_t n = static_cast<size_t>(samples);
   if (n == 0) return CUBLOX_OK;
@@ -1812,7 +1870,7 @@ static int fetch_copy(cublox_grid *g, cudaStream_t st, FetchScratch *sc, int64_t
     direct = true;
   }
   if (direct) CK(cudaStreamSynchronize(st));
-  return copy_out(g, st, sc, parts, bytes, 2);
+  return copy_out(g, st, parts, bytes, 2);
 }
 
 }  // extern "C"
@@ -1857,7 +1915,6 @@ void cublox_b200::detail::free_fetch(FetchScratch *sc) {
   cublox_b200::detail::dfree(sc->fpos);
   cublox_b200::detail::dfree(sc->fstate);
   cublox_b200::detail::hfree(sc->hoff);
-  cublox_b200::detail::hfree(sc->hcopy);
   *sc = FetchScratch{};
 }
 

@@ -27,8 +27,6 @@ struct FetchScratch {
   int64_t pending = -1;  // samples of a fetch_begin, still in fpos and fstate (-1: none)
   void *hoff = nullptr;  // pinned: the queries' offsets
   size_t hoff_bytes = 0;
-  void *hcopy = nullptr;  // pinned: samples on their way to pageable memory
-  size_t hcopy_bytes = 0;
 };
 // Bytes of one set of a map's line flags (16-byte loads start on its lines).
 inline size_t flag_bytes(int nlines) { return (static_cast<size_t>(nlines) + 255) & ~size_t(255); }
