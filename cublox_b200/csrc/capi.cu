@@ -1743,8 +1743,13 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
 // kIdle wait for the next one (several threads may copy at once).
 class StagingPool {
  public:
-  // A buffer (all have the same size), or null where there is no memory.
-  void *take(size_t bytes) {
+  static constexpr size_t kPiece = static_cast<size_t>(512) << 10;  // a thread's part of a buffer
+  static int threads() {
+    const int cores = static_cast<int>(std::thread::hardware_concurrency());
+    return std::max(1, std::min(8, cores / 2));
+  }
+  // A buffer of kPiece bytes per thread, or null where there is no memory.
+  void *take() {
     for (;;) {
       void *p = nullptr;
       {
@@ -1756,11 +1761,15 @@ class StagingPool {
       if (mem_kind(p) == 1) return p;  // else a device reset has freed it
     }
     void *p = nullptr;
-    if (cublox_b200::detail::hmalloc(&p, bytes) != cudaSuccess) {
+    if (cublox_b200::detail::hmalloc(&p, kPiece * threads()) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
     return p;
+  }
+  // Has a buffer wait for the next copy, if there is memory for one.
+  void reserve() {
+    if (void *p = take()) give(p);
   }
   void give(void *p) {
     {
@@ -1795,15 +1804,12 @@ static StagingPool &staging_pool() {
 static int copy_out(cublox_grid *g, cudaStream_t st,
                     const std::pair<const void *, void *> *parts, const size_t *bytes, int n_parts) {
   constexpr size_t kThreadedCopy = static_cast<size_t>(4) << 20;
-  constexpr size_t kPiece = static_cast<size_t>(512) << 10;
-  constexpr int kMostThreads = 8;
+  constexpr size_t kPiece = StagingPool::kPiece;
   size_t all = 0;
   for (int i = 0; i < n_parts; ++i)
     if (parts[i].second) all += bytes[i];
-  const int cores = static_cast<int>(std::thread::hardware_concurrency());
-  const int threads = std::max(1, std::min(kMostThreads, cores / 2));
-  char *stage =
-      all < kThreadedCopy ? nullptr : static_cast<char *>(staging_pool().take(kPiece * threads));
+  const int threads = StagingPool::threads();
+  char *stage = all < kThreadedCopy ? nullptr : static_cast<char *>(staging_pool().take());
   if (!stage) {
     for (int i = 0; i < n_parts; ++i)
       if (parts[i].second)
@@ -1889,10 +1895,8 @@ int cublox_b200::detail::fetch_into(cublox_grid *g, cudaStream_t st, const float
   if (n == 0) return CUBLOX_OK;
   char *dst = static_cast<char *>(room(13 * n));
   if (!dst) return fail(CUBLOX_ERR_NOMEM, "fetch: no memory for the samples");
-  CK(cudaMemcpyAsync(dst, sc->fpos, 12 * n, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(dst + 12 * n, sc->fstate, n, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  return CUBLOX_OK;
+  return fetch_copy(g, st, sc, total, reinterpret_cast<float *>(dst),
+                    reinterpret_cast<uint8_t *>(dst + 12 * n));
 }
 
 size_t cublox_b200::detail::fetch_block_bytes(int centres) {
@@ -1901,6 +1905,7 @@ size_t cublox_b200::detail::fetch_block_bytes(int centres) {
 
 int cublox_b200::detail::reserve_fetch(FetchScratch *sc, int centres, int64_t samples,
                                        cudaStream_t st) {
+  staging_pool().reserve();
   sc->fq_limit = fetch_block_bytes(centres);
   int rc = ensure_fq(sc, st, sc->fq_limit);
   if (!rc)

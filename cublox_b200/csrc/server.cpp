@@ -185,7 +185,7 @@ struct PinnedPool {
 // fit, and neighbours that are given back become one piece again.  A result
 // that finds no room is kept in pageable memory.
 struct ResultArena {
-  static constexpr size_t kMost = size_t(32) << 20, kGrain = size_t(4) << 10;
+  static constexpr size_t kGrain = size_t(4) << 10;
   std::mutex mu;
   char *base = nullptr;
   std::map<size_t, size_t> free;  // start, bytes
@@ -787,8 +787,10 @@ int cublox_server_create(const cublox_server_config *cfg, cublox_server **out) {
   if (!rc)
     rc = cublox_b200::detail::reserve_fetch(&s->fscratch, s->cfg.max_fetch_centres,
                                             s->cfg.max_fetch_samples, s->fstream);
-  if (!rc)
-    s->results.init(std::min<size_t>(ResultArena::kMost, s->cfg.pinned_pool_bytes / 8), s->device);
+  if (!rc)  // one result at the configured limit, or as many smaller ones
+    s->results.init(std::min<size_t>(s->cfg.pinned_pool_bytes / 4,
+                                     ResultArena::grains(13 * static_cast<size_t>(s->cfg.max_fetch_samples))),
+                    s->device);
   if (rc) {
     const std::string msg = cublox_last_error();
     cublox_b200::detail::free_fetch(&s->fscratch);

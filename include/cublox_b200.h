@@ -416,10 +416,11 @@ typedef struct cublox_server_config {
    * within these sizes allocates nothing (cublox_runtime_counters).        */
   uint64_t pinned_pool_bytes; /* pinned host arena that submitted scans are
                                  copied into (0: 256 MiB); a scan that finds
-                                 no room stays in pageable memory.  An eighth
-                                 as much more (32 MiB at most) holds results
-                                 of fetches until they are released; one that
-                                 finds no room is in pageable memory        */
+                                 no room stays in pageable memory.  Room for
+                                 max_fetch_samples more (a quarter as much at
+                                 most) holds results of fetches until they are
+                                 released; one that finds none is in pageable
+                                 memory                                     */
   int max_fetch_centres;      /* centres per fetch request (0: 1024)        */
   int64_t max_fetch_samples;  /* samples per fetch request (0: 1 << 22)     */
 } cublox_server_config;
