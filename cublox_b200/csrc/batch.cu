@@ -604,18 +604,24 @@ const Shape kShapes[] = {{0, 512, 512, 0, 1, 0, 0, 1},          {32, 1024, 1024,
                          {32, 512, 512, 2, 2, 0, 1, 0},         {32, 512, 512, 1, 2, 0, 1, 0},
                          {32, 1024, 512, 0, 2, 0, 1, 0},        {32, 768, 512, 0, 2, 0, 1, 0}};
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
-constexpr int kWideShape = 10;  // walks the maps that the cone walk does not take (cone_takes)
+// Walks the maps that the cone walk does not take (cone_takes), and the whole
+// batch beside one: 4 maps of 4201 x 61 x 41 230 us, with the tuner's choice
+// among ten shapes before that walk came in 229; one of them and 7 of 401 x 401
+// x 81 658 (730).
+constexpr int kWideShape = 10;
 
 // The tuner's candidates: the cone walk's item forms with the default voxel
-// layout (8 x 4 x 1 bricks), its usual one with 4 x 8 x 1 and 4 x 4 x 2
-// bricks, and the fastest of the shapes with a counter cube.  Two rays a
-// thread (shape 4: smaller CTAs, each warp a long row of rays and a short one)
-// suit batches of many items (32 maps of three sizes: walk 1.09 ms, shape 0
-// 1.20, shape 10 3.19), one ray a thread those of few (8 README-scale maps:
-// 0.73, 0.64, 1.16).  The other shapes and the reference's hash order have
-// not been the fastest on any workload measured and are not timed; all stay
-// selectable.  A candidate with another layout moves every grid of the update
-// to it first.
+// layout (8 x 4 x 1 bricks), its usual one with 4 x 8 x 1 and 4 x 4 x 2 bricks,
+// and the fastest of the shapes with a counter cube.  Of 12 batches (the listed
+// two of perf/cases.py and ten drawn ones) the 256-ray items were the fastest
+// for 8 (11 maps of 189 x 311 x 117 voxels and smaller: walk and fold 137 us,
+// 153 with 512), 512 rays, one a thread, for 2 (8 README-scale maps 1.07 ms,
+// 1.11) and two a thread for 2 (32 maps of three sizes 1.51 ms, 1.60).  The
+// other layouts were within 3 % of the fastest for one of them each, shape 10
+// for none (1.2 to 2.3 times as long); they are timed, twice each, for maps
+// and scans unlike these.  The remaining shapes and the reference's hash order
+// are not; all stay selectable.  A candidate with another layout moves every
+// grid of the update to it first.
 struct Candidate {
   int shape, layout;
 };

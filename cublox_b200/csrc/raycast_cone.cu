@@ -53,7 +53,9 @@ void launch(const RayParams &p, cudaStream_t s) {
 // 1,024 rays (the split walk with its plan: last): 16-beam scan of 16,384 rays
 // 32 / 37 / 39 / 46 / - (78); 64 beams, 65,536 rays 186 / 148 / 119 / 116 /
 // 179 (216); 128 beams, 262,144 rays 587 / 570 / 455 / 398 / 377 (933); 640 x
-// 480 depth image, 307,200 rays 68 / 61 / 63 / 68 / 74 (205).
+// 480 depth image, 307,200 rays 68 / 61 / 63 / 68 / 74 (205).  The rule takes
+// the fastest for the first of these and is 3 us, 21 and 7 off it for the
+// others: no size but 256 and 512 is near the fastest for both of the last two.
 void launch_raycast_cone(const RayParams &p, cudaStream_t s) {
   if (p.n <= 0) return;
   const int fit = p.n / 256;

@@ -111,12 +111,13 @@ int cublox_grid_get_fp_mode(const cublox_grid *g, unsigned *mode);
  * every choice, only speed differs).                                       */
 #define CUBLOX_OPT_RAYCAST 1 /* 0: one thread per ray; 1: direction-binned
                                 warp walk; 2 (default): 32 neighbouring
-                                rays per warp in step, or, for maps whose
-                                sides sum to more than 4,082 voxels and
-                                where CUBE, SORT, SEGMENT, BLOCK,
-                                CONTIGUOUS or FLAT_CUBE is not at its
-                                default, rays split between lanes at exact
-                                time cuts                                  */
+                                rays per warp in step, or rays split between
+                                lanes at exact time cuts: for maps whose
+                                sides sum to more than 4,082 voxels or that
+                                hold more than 2^29, for scans with rays so
+                                long and so few that it is faster, and where
+                                CUBE, SORT, SEGMENT, BLOCK, CONTIGUOUS or
+                                FLAT_CUBE is not at its default            */
 #define CUBLOX_OPT_CUBE 2    /* shared-memory counter cube side around the
                                 sensor: 0, 8, 16 or 32 (default 32; 8 is
                                 split walk only)                           */
