@@ -639,6 +639,7 @@ static bool cone_pays(const cublox_grid *g, int n, const float sensor[3]) {
   // a ray's steps are at most sqrt(3) times its length; few go far up or down
   const float level = far[0] + far[1];
   const float chain = std::min(level + std::min(far[2], level), 1.7321f * reach + 4.0f);
+  if (chain <= 710.0f) return true;
   const float a = std::max(near[0], near[1]), b = std::min(near[0], near[1]);
   const float t = std::atan2(b, a);  // azimuth of the window's corner
   const float mean = 0.6366f * (a * (t - std::log(std::cos(t))) +
@@ -1739,42 +1740,48 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
 }
 
 // Pinned staging buffers for copy_out, shared by all grids: pinning 4 MB takes
-// 2 to 4 ms, more than most fetches.  Each is used by one copy at a time; up to
-// kIdle wait for the next one (several threads may copy at once).
+// 2 to 4 ms, more than most fetches.  Each is used by one copy at a time, and
+// the one used longest ago comes next: a buffer that the CPU has just read takes
+// the device's writes more slowly (54 MB through one buffer 3.25 ms, through
+// kKept in turn 3.0).  The first kKept copies make one each; a copy that finds
+// all in use makes one that goes again.
 class StagingPool {
  public:
   static constexpr size_t kPiece = static_cast<size_t>(512) << 10;  // a thread's part of a buffer
-  static int threads() {
-    const int cores = static_cast<int>(std::thread::hardware_concurrency());
-    return std::max(1, std::min(8, cores / 2));
+  static int threads() {  // counted once: the count reads a file
+    static const int n =
+        std::max(1, std::min(8, static_cast<int>(std::thread::hardware_concurrency()) / 2));
+    return n;
   }
   // A buffer of kPiece bytes per thread, or null where there is no memory.
   void *take() {
-    for (;;) {
-      void *p = nullptr;
-      {
-        std::lock_guard<std::mutex> lk(mu_);
-        if (idle_.empty()) break;
-        p = idle_.back();
-        idle_.pop_back();
-      }
-      if (mem_kind(p) == 1) return p;  // else a device reset has freed it
+    bool more;
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      more = kept_ < kKept;
+      if (more) ++kept_;
     }
-    void *p = nullptr;
-    if (cublox_b200::detail::hmalloc(&p, kPiece * threads()) != cudaSuccess) {
+    void *p = more ? nullptr : idle();
+    if (!p && cublox_b200::detail::hmalloc(&p, kPiece * threads()) != cudaSuccess) {
       cudaGetLastError();
-      return nullptr;
+      if (more) {
+        std::lock_guard<std::mutex> lk(mu_);
+        --kept_;
+      }
+      p = more ? idle() : nullptr;
     }
     return p;
   }
   // Has a buffer wait for the next copy, if there is memory for one.
   void reserve() {
-    if (void *p = take()) give(p);
+    void *p = idle();
+    if (!p) p = take();
+    if (p) give(p);
   }
   void give(void *p) {
     {
       std::lock_guard<std::mutex> lk(mu_);
-      if (idle_.size() < kIdle) {
+      if (idle_.size() < kKept) {
         idle_.push_back(p);
         return;
       }
@@ -1783,9 +1790,21 @@ class StagingPool {
   }
 
  private:
-  static constexpr size_t kIdle = 2;
+  static constexpr size_t kKept = 3;
+  // The buffer that has waited longest, if any does.
+  void *idle() {
+    std::lock_guard<std::mutex> lk(mu_);
+    while (!idle_.empty()) {
+      void *p = idle_.front();
+      idle_.pop_front();
+      if (mem_kind(p) == 1) return p;
+      --kept_;  // a device reset has freed it
+    }
+    return nullptr;
+  }
   std::mutex mu_;
-  std::vector<void *> idle_;
+  std::deque<void *> idle_;
+  size_t kept_ = 0;  // made to be kept, in use or waiting
 };
 
 static StagingPool &staging_pool() {

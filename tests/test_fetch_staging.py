@@ -1,7 +1,7 @@
 """Large fetches into pageable memory, whose pinned staging buffers outlive the
-grids: a grid's first fetch pins none if an earlier grid's is there, fetches of
-several grids at once each have their own, and one that can have none still
-gets its samples."""
+grids: once three are there, a grid's first fetch pins none; fetches of several
+grids at once each have their own, and one that can have none still gets its
+samples."""
 import threading
 
 import numpy as np
@@ -33,7 +33,7 @@ def _alone(g, c):
 def test_staging_outlives_the_grid():
     c = _centres(150)  # 8 MB
     pinned = []
-    for seed in range(3):
+    for seed in range(6):
         g = _grid(seed)
         want = _alone(g, c)
         before = C.runtime_counters()["pinned_allocs"]
@@ -42,7 +42,7 @@ def test_staging_outlives_the_grid():
         assert pos.nbytes + st.nbytes > 4 << 20
         assert np.array_equal(pos, want[0]) and np.array_equal(st, want[1])
         g.close()
-    assert pinned[1:] == [0, 0], pinned
+    assert max(pinned) <= 1 and pinned[3:] == [0, 0, 0], pinned
 
 
 def test_grids_that_fetch_at_once():
@@ -63,7 +63,7 @@ def test_grids_that_fetch_at_once():
     for t in threads:
         t.join()
     assert not bad
-    # two buffers are kept; the other three grids' went back
+    # three buffers are kept; the other grids' went back
     n = C.runtime_counters()
     C.fail_allocations(0, 1 << 20)
     try:
