@@ -1099,13 +1099,18 @@ def main():
             "peak": h["peak"], "frac": fold_gbs / h["peak"], "peak_source": h["peak_kind"],
             "basis": "the fold's ncu DRAM bytes per map x maps / its live device time: the "
                      "bytes it must move (256 B read and up to 256 B written per flagged line)"}
-    out["roofline"]["l2_atomic"] = {
-        "kernel": "batch walk", "achieved": ach, "unit": "atomic adds/s",
-        "peak": red_l2, "frac": ach / red_l2, "peak_beyond_l2": red_hbm,
-        "peak_source": "cublox_probe_red_rate on this GPU, this run (distinct pseudo-random "
-                       "addresses; 64 MiB buffer in L2, and 4 GiB beyond it)",
-        "note": "effective: U + H in-window increments per walk time; the shared-memory "
-                "sensor cube takes part of them off the global atomics"}
+    requests = profiled_traffic(h["K"], "walk_red_requests_per_map")[0]
+    if requests:
+        rate = requests / (float(np.mean(h["walk_ms"])) / 1e3)
+        out["roofline"]["l2_atomic"] = {
+            "kernel": "batch walk", "achieved": rate, "unit": "reduction requests/s",
+            "peak": red_l2, "frac": rate / red_l2, "peak_beyond_l2": red_hbm,
+            "peak_source": "cublox_probe_red_rate on this GPU, this run (distinct pseudo-random "
+                           "addresses; 64 MiB buffer in L2, and 4 GiB beyond it)",
+            "increments_per_s": ach,
+            "basis": "the walk's ncu reduction requests at L2 per map (default launch shape) x maps "
+                     "/ its live device time; a request adds for all lanes on one voxel or in one "
+                     "sector, so the U + H in-window increments are about three a request"}
     if world == 1 and not args.only_headline:
         out["plain"] = run_plain(args, h)
         out["batching"] = run_batching(args)
