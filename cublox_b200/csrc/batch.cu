@@ -319,6 +319,8 @@ __device__ __forceinline__ FoldView fold_view(const MapDesc &m) {
                   m.l_unknown, m.ray.fp};
 }
 
+__device__ __forceinline__ uint8_t *hot_flags(const MapDesc &m) { return m.ray.dirty + m.ray.hot; }
+
 // One fold item: the flagged lines among [start, start + count), the CTA's
 // warps taking groups of 32 lines in turn.  kAll: fold every line of the
 // item, flagged or not (the reference's full sweep, for comparison).
@@ -326,7 +328,7 @@ template <bool kL2, bool kAll = false>
 __device__ __forceinline__ uint32_t fold_item(const MapDesc &m, const FoldItem &item) {
   const FoldView v = fold_view(m);
   const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  return fold_lines<8, kL2, kAll>(v, m.ray.dirty, m.ray.hot, item.start + 32 * warp, item.start + item.count,
+  return fold_lines<8, kL2, kAll>(v, m.ray.dirty, hot_flags(m), item.start + 32 * warp, item.start + item.count,
                                   32 * warps);
 }
 
@@ -468,8 +470,8 @@ __global__ void __launch_bounds__(kListThreads, kMinCtas) batch_fold_list_kernel
     const FoldItem item = items[s_item];
     const MapDesc &m = maps[item.map];
     const uint4 f = load_line_flags(m.ray.dirty, item.start, item.count);
-    const uint4 fh = load_line_flags(m.ray.hot, item.start, item.count);
-    const int2 n = build_line_list(line_flag_bits(f), line_flag_bits(fh), L, m.ray.dirty, m.ray.hot,
+    const uint4 fh = load_line_flags(hot_flags(m), item.start, item.count);
+    const int2 n = build_line_list(line_flag_bits(f), line_flag_bits(fh), L, m.ray.dirty, hot_flags(m),
                                    item.start, item.count);
     add_touched(m, fold_line_list<kQuads, false>(fold_view(m), L, n, item.start));
     __syncthreads();  // the list and s_item are rewritten next
@@ -574,8 +576,8 @@ __global__ void __launch_bounds__(512, 2) batch_fused_flat_kernel(const MapDesc 
       __syncthreads();
       if (s_ok) {
         const uint4 f = load_line_flags<true>(m.ray.dirty, item.start, item.count);
-        const uint4 fh = load_line_flags<true>(m.ray.hot, item.start, item.count);
-        const int2 n = build_line_list(line_flag_bits(f), line_flag_bits(fh), L, m.ray.dirty, m.ray.hot,
+        const uint4 fh = load_line_flags<true>(hot_flags(m), item.start, item.count);
+        const int2 n = build_line_list(line_flag_bits(f), line_flag_bits(fh), L, m.ray.dirty, hot_flags(m),
                                       item.start, item.count);
         add_touched(m, fold_line_list<2, true>(fold_view(m), L, n, item.start));
       }

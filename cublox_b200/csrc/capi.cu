@@ -685,7 +685,7 @@ static int integrate(cublox_grid *g, const float *dx, const float *dy,
   p.err = g->d_err;
   p.lay = g->lay;
   p.dirty = g->d_dirty;
-  p.hot = g->d_dirty + flag_bytes(g->nlines);
+  p.hot = static_cast<uint32_t>(flag_bytes(g->nlines));
   if ((g->opt_raycast == 1 || (g->opt_raycast == 2 && g->opt_sort)) && n > g->bin_cap) {
     CK(cudaStreamSynchronize(g->stream));
     cublox_b200::detail::dfree(g->d_bins);
@@ -826,7 +826,7 @@ RayParams cublox_b200::detail::ray_params(const cublox_grid *g, const float *x,
   p.err = g->d_err;
   p.lay = g->lay;
   p.dirty = g->d_dirty;
-  p.hot = g->d_dirty + flag_bytes(g->nlines);
+  p.hot = static_cast<uint32_t>(flag_bytes(g->nlines));
   return p;
 }
 

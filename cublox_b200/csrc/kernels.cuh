@@ -69,7 +69,7 @@ struct RayParams {
   uint32_t *err;
   VoxLayout lay;
   uint8_t *dirty;  // line flags to set, or null (the fold sweeps every line)
-  uint8_t *hot;    // flags of lines with a hit; null where dirty is
+  uint32_t hot;    // where the flags of lines with a hit start, after dirty
 };
 
 struct ApplyParams {

@@ -94,7 +94,7 @@ int fold(const cublox_map_view *map, const RayParams &p, int first, int n, int v
   a.stats = nullptr;
   a.variant = variant;
   a.dirty = p.dirty;
-  a.hot = p.hot;
+  a.hot = p.dirty ? p.dirty + p.hot : nullptr;
   a.nlines = lines;
   launch_apply(a, s);
   const cudaError_t e = cudaGetLastError();
@@ -207,7 +207,7 @@ int cublox_integrate_noalloc(const cublox_map_view *map, const float *xyz_soa, i
   p.lay.bs[0] = mapsz[1] * mapsz[2];
   p.lay.bs[1] = mapsz[2];
   p.lay.bs[2] = 1;
-  p.dirty = p.hot = nullptr;
+  p.dirty = nullptr;
 
   // lines of 32 voxels in full, and the last, partial one
   const int64_t lines = vnum >> kLineShift;
@@ -215,7 +215,7 @@ int cublox_integrate_noalloc(const cublox_map_view *map, const float *xyz_soa, i
   if (flags <= kFlagLines && cone_takes(mapsz, vnum) && aligned(map->occ, 16) &&
       aligned(map->cnt, 16) && aligned(map->hit, 16)) {
     p.dirty = base;
-    p.hot = base + flags;
+    p.hot = static_cast<uint32_t>(flags);
     if ((e = cudaMemsetAsync(base, 0, 2 * flags, s)) == cudaSuccess) {
       launch_raycast_cone(p, s);
       e = cudaGetLastError();

@@ -116,7 +116,7 @@ __device__ __forceinline__ void mark_line(const RayParams &p, int h, int &last) 
 __device__ __forceinline__ void mark_hit(const RayParams &p, int h, uint32_t hits) {
   atomicOr(p.cnt + h, kHitFlag);
   atomicAdd(p.hit + h, hits);
-  if (p.hot) p.hot[h >> kLineShift] = 1;
+  if (p.dirty) p.dirty[p.hot + static_cast<uint32_t>(h >> kLineShift)] = 1;
 }
 
 // One step, tie rule of kernels.cu:120-136.  Returns the axis stepped.
