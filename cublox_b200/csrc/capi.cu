@@ -1622,8 +1622,8 @@ static int fetch_run(cublox_grid *g, cudaStream_t st, const float *centers, int 
   // A server's block is small, and its outputs mostly empty: a fetch of several
   // groups has them in the second half of the outputs instead, and the samples
   // in the first, as long as they fit.
-  const size_t half = align256(sizeof(float) * 3 * static_cast<size_t>(sc->fcap) / 2);
-  const size_t upper = sizeof(float) * 3 * static_cast<size_t>(sc->fcap) - half;
+  const size_t out_bytes = sizeof(float) * 3 * static_cast<size_t>(sc->fcap);
+  const size_t half = align256(out_bytes / 2), upper = out_bytes - std::min(half, out_bytes);
   bool lent = sc->fq_limit && plan.groups.size() > 1 && upper > limit;
   if (lent) {
     plan.cut(upper);

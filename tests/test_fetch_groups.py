@@ -70,6 +70,27 @@ def test_served_fetches_of_any_radius_allocate_nothing():
     srv.close()
 
 
+@pytest.mark.parametrize("samples", [1, 1 << 18])
+def test_served_fetches_of_more_samples_than_configured(samples):
+    """Outputs too small to lend room to the block, and outputs whose lower half
+    a fetch's samples do not fit: they are found again beside the block."""
+    rng = np.random.default_rng(7)
+    p, s = _scan(rng, FLAT)
+    o = _oracle(FLAT, p, s)
+    for r, flt, cap, n in [(1.5, -1, 0, 64), (15.0, 1, 0, 2), (23.4, -1, 0, 1), (2.0, 2, 0, 64), (23.4, 1, 0, 3)]:
+        srv = C.Server(hbm_budget_bytes=1 << 30, max_tick_points=1 << 16, max_fetch_centres=64,
+                       max_fetch_samples=samples, pinned_pool_bytes=1 << 24)
+        mid = srv.add_map(FLAT, 0.1, False, None, max_range=30.0, log_odds=LO)
+        assert srv.wait(srv.submit_scan(mid, p, s, False)) == C.REQ_DONE
+        centres = (s + rng.uniform(-3, 3, (n, 3)) * [1, 1, 0.05]).astype(np.float32)
+        centres[0] = s
+        for _ in range(2):  # with room to make, and with room made
+            rid = srv.submit_fetch(mid, centres, r, None if flt < 0 else flt, cap)
+            assert srv.wait(rid) == C.REQ_DONE
+            _same(o, centres, r, flt, cap, *srv.fetch_result(rid, n))
+        srv.close()
+
+
 def test_a_grids_block_is_bounded_and_small_where_memory_is_short():
     import torch
 
