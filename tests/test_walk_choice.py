@@ -76,3 +76,22 @@ def test_sensors_and_ranges_at_the_ends(s, max_range):
     o.update(p, np.float32(s))
     assert np.array_equal(g.export().view(np.uint32), o.occ().view(np.uint32))
     g.close()
+
+
+@pytest.mark.parametrize("away", [30.0, 2e4, 1e5])
+def test_sensor_far_outside_the_window(away):
+    """Rays that reach the window after 100 steps, or after hundreds of thousands."""
+    half, rng = (30, 25, 8), np.random.default_rng(int(away))
+    g, o = C.OccupancyGrid(half, 0.1, False, None), O.OracleGrid(half, 0.1, False, None)
+    s = np.float32([away, 0.03, 0.05])
+    p = (rng.normal(size=(200, 3)) * [1.5, 1.0, 0.4]).astype(np.float32)
+    for x, lo, mr in ((g, g.setLogOddsParams, g.setMaxRaycastRange), (o, o.set_log_odds, o.set_max_range)):
+        lo(*LO)
+        mr(3e38)
+        x.set_origin_index((0, 0, 0))
+    g.update(p, s)
+    o.update(p, s)
+    assert np.count_nonzero(o.occ()) > 200
+    assert np.array_equal(g.export().view(np.uint32), o.occ().view(np.uint32))
+    assert g.check() == 0
+    g.close()
